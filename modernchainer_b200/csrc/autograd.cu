@@ -728,7 +728,14 @@ static mcb_status linear_backward_impl(mcb_ctx *ctx, const Tensor &g_in, const L
             MCB_TRY(to_dtype(ctx, w->data, sv.lp, &t));
             MCB_TRY(to_dtype(ctx, t, MCB_F32, &wf));
         }
-        MCB_TRY(mcb_linear_backward(ctx, (const float *)g.ptr, (const float *)sv.x.ptr, (const float *)wf.ptr, dx, dw, nullptr, m, k, n));
+        float *db = nullptr;
+        if (want_db && dw) { // the weight-gradient product reads the whole gradient anyway: it leaves the column sums
+            bool direct;
+            MCB_TRY(grad_dst(b, &gi[2], &direct));
+            db = (float *)gi[2].ptr;
+            db_done = true;
+        }
+        MCB_TRY(mcb_linear_backward(ctx, (const float *)g.ptr, (const float *)sv.x.ptr, (const float *)wf.ptr, dx, dw, db, m, k, n));
         if (x->requires_grad && is_lp(x->data.dt)) {
             Tensor t;
             MCB_TRY(to_dtype(ctx, gi[0], x->data.dt, &t));
@@ -795,13 +802,8 @@ static mcb_status f_linear_impl(const Var &x, const Var &w, const Var &b, int ac
         }
         MCB_TRY(new_tensor(ctx, MCB_F32, oshape, &res));
         const float *bp = b ? (const float *)b->data.ptr : nullptr;
-        if (act != MCB_ACT_NONE) {
-            MCB_TRY(new_tensor(ctx, MCB_F32, oshape, &sv->pre));
-            MCB_TRY(mcb_linear(ctx, (const float *)sv->x.ptr, (const float *)wf.ptr, bp, (float *)sv->pre.ptr, m, k, n, MCB_ACT_NONE));
-            MCB_TRY((act == MCB_ACT_GELU ? mcb_gelu : mcb_relu)(ctx, sv->pre.ptr, res.ptr, res.numel(), MCB_F32));
-        } else {
-            MCB_TRY(mcb_linear(ctx, (const float *)sv->x.ptr, (const float *)wf.ptr, bp, (float *)res.ptr, m, k, n, MCB_ACT_NONE));
-        }
+        if (act != MCB_ACT_NONE) MCB_TRY(new_tensor(ctx, MCB_F32, oshape, &sv->pre));
+        MCB_TRY(mcb_linear_pre(ctx, (const float *)sv->x.ptr, (const float *)wf.ptr, bp, (float *)res.ptr, (float *)sv->pre.ptr, m, k, n, act));
         if (sv->emulated) { // stored like the tensor-core path stores it: result in the 16-bit type, pre-activation rounded to it
             Tensor t;
             MCB_TRY(to_dtype(ctx, res, lp, &t));

@@ -168,6 +168,44 @@ static inline cudaError_t mcb_launch_dep(mcb_ctx *ctx, void (*kernel)(KArgs...),
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// raises a kernel's dynamic shared-memory limit to `bytes`, once per kernel and device (always call it with the same bytes)
+template <typename... KArgs> static inline cudaError_t mcb_smem_limit(mcb_ctx *ctx, void (*kernel)(KArgs...), size_t bytes) {
+    static std::mutex mu;
+    static std::unordered_map<void *, unsigned long long> done; // per kernel, one bit per device
+    std::lock_guard<std::mutex> lk(mu);
+    unsigned long long &bits = done[(void *)kernel];
+    const unsigned long long bit = 1ull << (ctx->device & 63);
+    if (bits & bit) return cudaSuccess;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e == cudaSuccess) bits |= bit;
+    return e;
+}
+
+// the same with a thread-block cluster (a cluster of one CTA is an ordinary launch)
+template <typename... KArgs, typename... Args>
+static inline cudaError_t mcb_launch_dep_cluster(mcb_ctx *ctx, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, dim3 cluster, Args &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    if (ctx->dep_launch) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster.x * cluster.y * cluster.z > 1) {
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = cluster.x;
+        at[n].val.clusterDim.y = cluster.y;
+        at[n++].val.clusterDim.z = cluster.z;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // ------------------------------------------------------------------ device helpers
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

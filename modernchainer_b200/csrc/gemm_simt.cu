@@ -1,118 +1,204 @@
-// Exact-f32 GEMM family (FFMA, no tensor cores): the MCB_COMPUTE_F32 path behind
+// Exact-f32 GEMM family (packed f32 FMAs, no tensor cores): the MCB_COMPUTE_F32 path behind
 // Ops::matmul / linear / linear_backward, and the batched products of the f32 attention.
 // One kernel with generic element strides covers NN / NT / TN operands, so no transpose is
 // ever materialised (the reference builds grad^T with transpose2d_f32 in every
 // linear_backward, crates/modern-chainer-cuda/src/ops.rs:833-843).
+//
+// Bound by the FMA pipe for large products and by latency for the small ones a training step of an f32 model is made of:
+// three or four stages of cp.async keep the loads of the coming slabs in flight, groups of threads inside a CTA and the CTAs of
+// a thread-block cluster take slices of the reduction, and their partial tiles are added through (distributed) shared memory in
+// a fixed order (same bits every run), so a split product is one launch without a workspace.  Measured (warm, back to
+// back), a 64 x 64 tile with one slab in registers -> this kernel: 1600 x 256 x 256 25 -> 13 us, 128 x 784 x 100 12 (two
+// launches) -> 6.5 us, 4096^3 from about 15 to 44 (x w^T) ... 54 (g^T x) TFLOP/s.
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
 #include "internal.h"
+#include "simt_tile.cuh"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4, kThreads = 256;
+using namespace simt;
 
-__global__ void __launch_bounds__(kThreads) sgemm_kernel(SgemmParams p) {
-    __shared__ float As[BK][BM + 4];
-    __shared__ float Bs[BK][BN + 4];
-    int bz = blockIdx.z;
-    long long bo = bz / p.batch_inner, bi = bz % p.batch_inner;
+__device__ __forceinline__ float gelu_f32(float v) {
+    float v3 = v * v * v;
+    return 0.5f * v * (1.0f + tanhf(0.7978845608028654f * (v + 0.044715f * v3)));
+}
+
+struct Epilogue {
+    float *C, *pre;
+    __device__ __forceinline__ void store(const SgemmParams &p, long long gi, long long gj, float v) const {
+        v *= p.alpha;
+        if (p.bias) v += p.bias[gj];
+        const long long at = gi * p.ldc + gj;
+        if (pre) pre[at] = v;
+        if (p.act == MCB_ACT_RELU) v = v > 0.0f ? v : 0.0f;
+        else if (p.act == MCB_ACT_GELU) v = gelu_f32(v);
+        C[at] = p.accumulate ? (C[at] + v) : v;
+    }
+};
+
+template <int BM, int BN, int TM, int TN, bool AKC, bool BKC, int STAGES, int G>
+__global__ void __launch_bounds__(G * (BM / TM) * (BN / TN)) sgemm_kernel(const SgemmParams p) {
+    using T = Tile<BM, BN, TM, TN, AKC, BKC>;
+    constexpr int NT = T::kThreads;
+    extern __shared__ __align__(16) float smem[];
+    const int splits = p.splits;
+    const int slice = splits > 1 ? (int)(blockIdx.z % splits) : 0;
+    const long long bz = blockIdx.z / splits, bo = bz / p.batch_inner, bi = bz % p.batch_inner;
     const float *A = p.a + bo * p.a_bo + bi * p.a_bi;
     const float *B = p.b + bo * p.b_bo + bi * p.b_bi;
-    float *C = p.c + bo * p.c_bo + bi * p.c_bi;
-    int tid = threadIdx.x;
-    int tx = tid % (BN / TN), ty = tid / (BN / TN);
-    long long m0 = (long long)blockIdx.y * BM, n0 = (long long)blockIdx.x * BN;
-    // split reduction (single problems that would fill only a few SMs): slice blockIdx.z of the k range, partial result to a
-    // workspace of p.splits [m, n] matrices that sgemm_reduce_kernel adds in slice order
-    long long k_begin = 0, k_end = p.k;
-    if (p.splits > 1) {
-        const long long per = ((p.k + p.splits - 1) / p.splits + BK - 1) / BK * BK;
-        k_begin = (long long)bz * per;
-        k_end = k_begin + per < p.k ? k_begin + per : p.k;
-        A = p.a;
-        B = p.b;
-        C = p.ws + (long long)bz * p.m * p.n;
+    const long long c_off = bo * p.c_bo + bi * p.c_bi;
+    const Epilogue epi{p.c + c_off, p.c_pre ? p.c_pre + c_off : nullptr};
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN, M = (int)p.m, N = (int)p.n, K = (int)p.k;
+    // every group of NT threads takes a slice of the reduction of its own (whole slabs), with its own stages and barrier
+    const int group = threadIdx.x / NT, tid = threadIdx.x % NT;
+    const int slabs = (K + BK - 1) / BK, per = (slabs + splits * G - 1) / (splits * G);
+    const int k_begin = min(K, (slice * G + group) * per * BK), k_end = min(K, k_begin + per * BK);
+    const int nk = (k_end - k_begin + BK - 1) / BK;
+    float *stage = smem + group * STAGES * T::kStageFloats;
+    T t;
+    t.init(tid);
+    const bool want_rowsum = !AKC && p.rowsum && blockIdx.x == 0;
+    float rsum[(BM + NT - 1) / NT] = {};
+    dep_wait();
+    dep_trigger();
+    auto fetch = [&](int s) {
+        if (s < nk) {
+            float *as = stage + (s % STAGES) * T::kStageFloats;
+            load_tile<BM, NT, AKC>(as, A, p.as0, p.as1, m0, M, k_begin + s * BK, k_end, p.a_vec, tid);
+            load_tile<BN, NT, BKC>(as + T::kAFloats, B, p.bs1, p.bs0, n0, N, k_begin + s * BK, k_end, p.b_vec, tid);
+        }
+        cp_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) fetch(s);
+    for (int s = 0; s < nk; ++s) {
+        cp_wait<STAGES - 2>();
+        if (G == 1) __syncthreads(); // slab s has landed for everybody, and everybody is done with the stage the next fetch overwrites
+        else group_sync(1 + group, NT);
+        fetch(s + STAGES - 1);
+        const float *as = stage + (s % STAGES) * T::kStageFloats;
+        t.mma(as, as + T::kAFloats);
+        if constexpr (!AKC) {
+            if (want_rowsum) { // sums of A over the reduction (a bias gradient), from the slab that is here anyway
+#pragma unroll
+                for (int h = 0; h < (BM + NT - 1) / NT; ++h) {
+                    const int r = tid + h * NT;
+                    float v = 0.0f;
+                    if (r < BM)
+#pragma unroll
+                        for (int k = 0; k < BK; ++k) v += as[k * (BM + 4) + r];
+                    rsum[h] += v;
+                }
+            }
+        }
     }
-    float acc[TM][TN];
+    cp_wait<0>();
+    if (G == 1 && splits == 1) {
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int gi = m0 + t.row(i);
+            if (gi >= M) continue;
+#pragma unroll
+            for (int j = 0; j < TN; ++j) {
+                const int gj = n0 + t.col(j);
+                if (gj < N) epi.store(p, gi, gj, t.value(i, j));
+            }
+        }
+        if (want_rowsum && tid < BM && m0 + tid < M) p.rowsum[m0 + tid] = rsum[0];
+        return;
+    }
+    // The partial tiles of the groups, then of the cluster's CTAs, meet in (distributed) shared memory; CTA r of the cluster
+    // finishes its share of the rows.  Group order, then rank order: same bits every run.
+    constexpr int RP = BN + 4, PART = BM * RP + BM;
+    __syncthreads();
+    float *part = smem + group * PART;
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = 0.0f;
-
-    bool a_k_contig = (p.as1 == 1), b_n_contig = (p.bs1 == 1);
-    for (long long k0 = k_begin; k0 < k_end; k0 += BK) {
+        for (int j = 0; j < TN; ++j) part[t.row(i) * RP + t.col(j)] = t.value(i, j);
 #pragma unroll
-        for (int l = 0; l < (BM * BK) / kThreads; ++l) {
-            int e = tid + l * kThreads;
-            int i, d;
-            if (a_k_contig) { d = e % BK; i = e / BK; } else { i = e % BM; d = e / BM; }
-            long long gi = m0 + i, gd = k0 + d;
-            As[d][i] = (gi < p.m && gd < k_end) ? A[gi * p.as0 + gd * p.as1] : 0.0f;
+    for (int h = 0; h < (BM + NT - 1) / NT; ++h)
+        if (tid + h * NT < BM) part[BM * RP + tid + h * NT] = rsum[h];
+    if (splits > 1) cluster_sync();
+    else __syncthreads();
+    const unsigned mine = smem_u32(smem);
+    auto total = [&](int at) {
+        float v = 0.0f;
+        if (splits == 1) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) v += smem[g * PART + at];
+        } else {
+            for (int s = 0; s < splits; ++s) {
+                const unsigned peer = peer_addr(mine, s);
+#pragma unroll
+                for (int g = 0; g < G; ++g) v += peer_ld(peer + (unsigned)(g * PART + at) * 4);
+            }
         }
-#pragma unroll
-        for (int l = 0; l < (BN * BK) / kThreads; ++l) {
-            int e = tid + l * kThreads;
-            int j, d;
-            if (b_n_contig) { j = e % BN; d = e / BN; } else { d = e % BK; j = e / BK; }
-            long long gj = n0 + j, gd = k0 + d;
-            Bs[d][j] = (gj < p.n && gd < k_end) ? B[gd * p.bs0 + gj * p.bs1] : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int d = 0; d < BK; ++d) {
-            float a[TM], b[TN];
-#pragma unroll
-            for (int i = 0; i < TM; ++i) a[i] = As[d][ty * TM + i];
-#pragma unroll
-            for (int j = 0; j < TN; ++j) b[j] = Bs[d][tx * TN + j];
-#pragma unroll
-            for (int i = 0; i < TM; ++i)
-#pragma unroll
-                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-        }
-        __syncthreads();
+        return v;
+    };
+    const int rows = BM / splits, r_first = slice * rows;
+    for (int e = threadIdx.x; e < rows * BN; e += NT * G) {
+        const int r = r_first + e / BN, c = e % BN;
+        if (m0 + r < M && n0 + c < N) epi.store(p, m0 + r, n0 + c, total(r * RP + c));
     }
-#pragma unroll
-    for (int i = 0; i < TM; ++i) {
-        long long gi = m0 + ty * TM + i;
-        if (gi >= p.m) continue;
-#pragma unroll
-        for (int j = 0; j < TN; ++j) {
-            long long gj = n0 + tx * TN + j;
-            if (gj >= p.n) continue;
-            if (p.splits > 1) { // raw partial sum; scale, bias and activation follow the reduction
-                C[gi * p.n + gj] = acc[i][j];
-                continue;
+    if (want_rowsum)
+        for (int r = r_first + threadIdx.x; r < r_first + rows; r += NT * G)
+            if (m0 + r < M) p.rowsum[m0 + r] = total(BM * RP + r);
+    if (splits > 1) cluster_sync(); // nobody leaves while a peer still reads its tile
+}
+
+template <int BM, int BN, int TM, int TN, bool AKC, bool BKC, int STAGES, int G>
+mcb_status launch(mcb_ctx *ctx, const SgemmParams &p) {
+    using T = Tile<BM, BN, TM, TN, AKC, BKC>;
+    static_assert(BM <= T::kThreads || G > 1, "one row sum per thread");
+    auto kernel = sgemm_kernel<BM, BN, TM, TN, AKC, BKC, STAGES, G>;
+    constexpr size_t bytes = sizeof(float) * G * std::max(STAGES * T::kStageFloats, BM * (BN + 4) + BM);
+    MCB_CUDA(ctx, mcb_smem_limit(ctx, kernel, bytes));
+    dim3 grid((unsigned)((p.n + BN - 1) / BN), (unsigned)((p.m + BM - 1) / BM), (unsigned)(p.batch * p.splits));
+    MCB_CUDA(ctx, mcb_launch_dep_cluster(ctx, kernel, grid, dim3(T::kThreads * G), bytes, dim3(1, 1, (unsigned)p.splits), p));
+    ctx->launches++;
+    return MCB_OK;
+}
+
+template <bool AKC, bool BKC> mcb_status launch_tile(mcb_ctx *ctx, const SgemmParams &p, int tile) {
+    if (tile == 2) return launch<128, 64, 8, 8, AKC, BKC, 3, 1>(ctx, p);
+    if (tile == 1) return launch<64, 64, 8, 8, AKC, BKC, 3, 2>(ctx, p);
+    return launch<32, 32, 4, 4, AKC, BKC, 4, 4>(ctx, p);
+}
+
+// Tile and reduction split by a cost model in microseconds, fitted to every tile and split of 36 products from 128 x 10 x 100 to
+// 4096^3 (it picks within 2% of the fastest on average): a CTA takes `alone` per slab of its groups while it has an SM to
+// itself, another resident CTA adds `shared` per slab, and every CTA pays for its prologue and epilogue (more when its
+// partial tile meets others in the cluster).
+void plan(mcb_ctx *ctx, const SgemmParams &p, int *tile_out, int *split_out) {
+    static const struct { int bm, bn, slab; double alone, shared, cta, cta_split; } cfg[3] = {
+        {32, 32, 64, 0.87, 0.59, 0.8, 1.2}, {64, 64, 32, 1.46, 0.79, 3.0, 3.0}, {128, 64, 16, 1.48, 0.77, 4.4, 4.4}};
+    double best = 0.0;
+    *tile_out = 1;
+    *split_out = 1;
+    for (int c = 0; c < 3; ++c) {
+        const long long mt = (p.m + cfg[c].bm - 1) / cfg[c].bm, tiles = mt * ((p.n + cfg[c].bn - 1) / cfg[c].bn) * p.batch;
+        if (mt > 65535) continue;
+        for (int s = 1; s <= 8; s *= 2) {
+            if (s > 1 && (knob_on(ctx, K_SGEMM_NO_SPLIT) || p.k <= (s / 2) * cfg[c].slab || p.batch * s > 65535)) break;
+            const double per = (double)((p.k + cfg[c].slab * s - 1) / (cfg[c].slab * s));
+            double waves = (double)(tiles * s) / ctx->sm_count;
+            waves = waves < 4.0 ? std::ceil(waves) : waves + 0.5;
+            const double t = per * (cfg[c].alone + (waves - 1.0) * cfg[c].shared) + waves * (s == 1 ? cfg[c].cta : cfg[c].cta_split + 0.1 * s);
+            if (best == 0.0 || t < best) {
+                best = t;
+                *tile_out = c;
+                *split_out = s;
             }
-            float v = acc[i][j] * p.alpha;
-            if (p.bias) v += p.bias[gj];
-            if (p.act == MCB_ACT_RELU) v = v > 0.0f ? v : 0.0f;
-            else if (p.act == MCB_ACT_GELU) {
-                float v3 = v * v * v;
-                v = 0.5f * v * (1.0f + tanhf(0.7978845608028654f * (v + 0.044715f * v3)));
-            }
-            float *dst = C + gi * p.ldc + gj;
-            *dst = p.accumulate ? (*dst + v) : v;
         }
     }
 }
 
-__global__ void sgemm_reduce_kernel(SgemmParams p) {
-    long long total = p.m * p.n;
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
-    for (; i < total; i += stride) {
-        float v = 0.0f;
-        for (int s = 0; s < p.splits; ++s) v += p.ws[(long long)s * total + i]; // fixed order: same bits every run
-        v *= p.alpha;
-        const long long gi = i / p.n, gj = i - gi * p.n;
-        if (p.bias) v += p.bias[gj];
-        if (p.act == MCB_ACT_RELU) v = v > 0.0f ? v : 0.0f;
-        else if (p.act == MCB_ACT_GELU) {
-            float v3 = v * v * v;
-            v = 0.5f * v * (1.0f + tanhf(0.7978845608028654f * (v + 0.044715f * v3)));
-        }
-        float *dst = p.c + gi * p.ldc + gj;
-        *dst = p.accumulate ? (*dst + v) : v;
-    }
+bool vec_ok(const float *base, long long s0, long long s1, long long bo, long long bi) {
+    return mcb_aligned16(base) && ((s0 == 1 ? s1 : s0) % 4 == 0) && bo % 4 == 0 && bi % 4 == 0;
 }
 
 } // namespace
@@ -121,32 +207,22 @@ mcb_status mcb_sgemm(mcb_ctx *ctx, const SgemmParams &p_in) {
     SgemmParams p = p_in;
     if (p.m == 0 || p.n == 0 || p.batch == 0) return MCB_OK;
     if (p.batch > 65535) return mcb_fail(ctx, MCB_UNSUPPORTED, "sgemm batch > 65535");
+    if (p.m > INT32_MAX - 256 || p.n > INT32_MAX - 256 || p.k > INT32_MAX - 256) return mcb_fail(ctx, MCB_UNSUPPORTED, "sgemm extent above 2^31");
     ProfScope prof(ctx, MCB_PROF_GEMM_F32, 2.0 * (double)p.m * (double)p.n * (double)p.k * (double)p.batch,
                    4.0 * (double)p.batch * ((double)p.m * p.k + (double)p.n * p.k + (double)p.m * p.n));
-    dim3 grid((unsigned)((p.n + BN - 1) / BN), (unsigned)((p.m + BM - 1) / BM), (unsigned)p.batch);
-    // A single skinny product (a classifier head, a weight gradient with few rows) would occupy a handful of SMs for the
-    // whole reduction: cut the reduction into slices, one block each, and add the slices afterwards in a fixed order.
-    const long long tiles = (long long)grid.x * grid.y;
-    p.splits = 1;
-    if (p.batch == 1 && tiles * 2 <= ctx->sm_count && p.k >= 512 && !knob_on(ctx, K_SGEMM_NO_SPLIT)) {
-        long long s = (2ll * ctx->sm_count) / tiles;
-        if (s > p.k / 128) s = p.k / 128;
-        if (s > 64) s = 64;
-        if (s >= 2) {
-            void *ws;
-            MCB_TRY(mcb_scratch(ctx, sizeof(float) * (size_t)s * (size_t)p.m * (size_t)p.n, &ws));
-            p.splits = (int)s;
-            p.ws = (float *)ws;
-            grid.z = (unsigned)s;
-        }
-    }
-    sgemm_kernel<<<grid, kThreads, 0, ctx->stream>>>(p);
-    MCB_LAUNCHED(ctx);
-    if (p.splits > 1) {
-        sgemm_reduce_kernel<<<mcb_grid_for(ctx, p.m * p.n, 256, 4), 256, 0, ctx->stream>>>(p);
-        MCB_LAUNCHED(ctx);
-    }
-    return MCB_OK;
+    const bool akc = p.as1 == 1, bkc = p.bs0 == 1 && p.bs1 != 1;
+    if ((!akc && p.as0 != 1) || (!bkc && p.bs1 != 1)) return mcb_fail(ctx, MCB_UNSUPPORTED, "sgemm: an operand has no unit stride");
+    if (p.rowsum && akc) return mcb_fail(ctx, MCB_UNSUPPORTED, "sgemm: row sums need A with unit row stride");
+    p.a_vec = vec_ok(p.a, p.as0, p.as1, p.a_bo, p.a_bi);
+    p.b_vec = vec_ok(p.b, p.bs0, p.bs1, p.b_bo, p.b_bi);
+    int tile = 1;
+    plan(ctx, p, &tile, &p.splits);
+    if ((p.m + 63) / 64 > 65535) tile = 2;
+    if ((p.m + 127) / 128 > 65535) return mcb_fail(ctx, MCB_UNSUPPORTED, "sgemm: more than 8388480 rows");
+    if (akc && bkc) return launch_tile<true, true>(ctx, p, tile);
+    if (akc) return launch_tile<true, false>(ctx, p, tile);
+    if (bkc) return launch_tile<false, true>(ctx, p, tile);
+    return launch_tile<false, false>(ctx, p, tile);
 }
 
 static SgemmParams plain(const float *a, long long as0, long long as1, const float *b, long long bs0, long long bs1,
@@ -169,19 +245,30 @@ mcb_status mcb_matmul(mcb_ctx *ctx, const float *a, const float *b, float *c, in
 mcb_status mcb_linear(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *y, int64_t m,
                       int64_t k, int64_t n, int32_t act) {
     MCB_CHECK_CTX(ctx);
-    SgemmParams p = plain(x, k, 1, w, 1, k, y, m, n, k);
-    p.bias = bias;
-    p.act = act;
-    return mcb_sgemm(ctx, p);
+    return mcb_linear_pre(ctx, x, w, bias, y, nullptr, m, k, n, act);
 }
 
 mcb_status mcb_linear_backward(mcb_ctx *ctx, const float *g, const float *x, const float *w, float *dx, float *dw,
                                float *db, int64_t m, int64_t k, int64_t n) {
     MCB_CHECK_CTX(ctx);
     if (dx) MCB_TRY(mcb_sgemm(ctx, plain(g, n, 1, w, k, 1, dx, m, k, n)));      // dx[m,k] = g[m,n] w[n,k]
-    if (dw) MCB_TRY(mcb_sgemm(ctx, plain(g, 1, n, x, k, 1, dw, n, k, m)));      // dw[n,k] = g^T[n,m] x[m,k]
+    if (dw) {                                                                   // dw[n,k] = g^T[n,m] x[m,k], db = row sums of g^T
+        SgemmParams p = plain(g, 1, n, x, k, 1, dw, n, k, m);
+        if (n > 1 && k > 0 && m > 0) p.rowsum = db;
+        MCB_TRY(mcb_sgemm(ctx, p));
+        if (p.rowsum) return MCB_OK;
+    }
     if (db) MCB_TRY(mcb_col_sum(ctx, g, MCB_F32, m, n, db));
     return MCB_OK;
 }
 
 } // extern "C"
+
+mcb_status mcb_linear_pre(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *y, float *pre, int64_t m, int64_t k, int64_t n,
+                          int32_t act) {
+    SgemmParams p = plain(x, k, 1, w, 1, k, y, m, n, k);
+    p.bias = bias;
+    p.act = act;
+    p.c_pre = pre;
+    return mcb_sgemm(ctx, p);
+}

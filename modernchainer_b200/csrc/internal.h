@@ -17,11 +17,16 @@ struct SgemmParams {
     float alpha = 1.0f;
     int act = MCB_ACT_NONE;
     int accumulate = 0;
-    // set by mcb_sgemm, not by callers: reduction slices and their workspace (splits x [m, n])
+    float *c_pre = nullptr;  // optional second output: the value before the activation (same layout as c)
+    float *rowsum = nullptr; // optional [m]: sums of A over the reduction; A must have unit row stride (as0 == 1 != as1), batch 1
+    // set by mcb_sgemm, not by callers: reduction slices (one cluster CTA each), 16-byte copies legal
     int splits = 1;
-    float *ws = nullptr;
+    bool a_vec = false, b_vec = false;
 };
 mcb_status mcb_sgemm(mcb_ctx *ctx, const SgemmParams &p);
+// y = act(x w^T + bias) in f32, the pre-activation left in `pre` (may be NULL) by the same launch
+mcb_status mcb_linear_pre(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *y, float *pre, int64_t m, int64_t k, int64_t n,
+                          int32_t act);
 
 // Tensor-core GEMM with explicit leading dimensions and (sample, head) batching; see gemm_tc.cu.
 struct TcGemmParams {

@@ -1,0 +1,214 @@
+// The f32 FMA tile shared by the exact-f32 GEMM (gemm_simt.cu) and the direct convolutions (conv.cu): operand tiles in
+// shared memory filled by cp.async, a TM x TN register tile per thread, packed f32x2 FMAs.
+//
+// An operand tile is kept the way it lies in memory, so that filling it is 16-byte asynchronous copies with no
+// transposition:
+//   KC = true:  the reduction index is contiguous: [MN][KP], rows of BK floats padded to KP = 20 (80 bytes: the eight rows a
+//               128-bit load phase touches fall into eight different 16-byte bank groups)
+//   KC = false: the row / column index is contiguous: [BK][MN + 4]
+// A thread's rows (columns) are strided over the tile for KC and come in groups of four for the other layout; either way one
+// 128-bit shared-memory load brings four operand values.
+#pragma once
+#include "common.cuh"
+
+namespace simt {
+
+constexpr int BK = 16;
+constexpr int KP = BK + 4;
+
+__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
+// 16- and 4-byte asynchronous copies that read `bytes` (0 .. size) and fill the rest with zeros
+__device__ __forceinline__ void cp16(unsigned dst, const void *src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp4(unsigned dst, const void *src, int bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// two f32 FMAs, each rounded as fmaf rounds it
+__device__ __forceinline__ void fma2(unsigned long long &d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ void group_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ float comp(const float4 &v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
+
+template <int BM_, int BN_, int TM_, int TN_, bool AKC_, bool BKC_> struct Tile {
+    static constexpr int BM = BM_, BN = BN_, TM = TM_, TN = TN_;
+    static constexpr bool AKC = AKC_, BKC = BKC_;
+    static constexpr int TX = BN / TN, TY = BM / TM, kThreads = TX * TY;
+    static constexpr int kAFloats = AKC ? BM * KP : BK * (BM + 4);
+    static constexpr int kBFloats = BKC ? BN * KP : BK * (BN + 4);
+    static constexpr int kStageFloats = kAFloats + kBFloats;
+    static_assert(TX % 8 == 0 && TY % 4 == 0, "a warp covers 8 x 4 threads");
+
+    // Two FMAs per instruction need operand pairs in adjacent registers.  Where B's columns are contiguous the pair is two
+    // columns (A is duplicated); where both operands are contiguous along the reduction it is two steps of k, straight from
+    // the 128-bit loads: each accumulator is then an even-k and an odd-k sum that meet at the end.
+    static constexpr bool KPAIR = AKC && BKC;
+    static constexpr int NACC = KPAIR ? TN : TN / 2;
+
+    int tx, ty;
+    unsigned long long acc[TM][NACC];
+
+    __device__ __forceinline__ void init(int tid) {
+        const int warp = tid >> 5, lane = tid & 31;
+        constexpr int wx = TX / 8;
+        tx = (lane & 7) + 8 * (warp % wx);
+        ty = (lane >> 3) + 4 * (warp / wx);
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+            for (int j = 0; j < NACC; ++j) acc[i][j] = 0ull;
+    }
+    // tile coordinates of this thread's i-th row and j-th column
+    __device__ __forceinline__ int row(int i) const { return AKC ? ty + i * TY : (i / 4) * (4 * TY) + ty * 4 + (i & 3); }
+    __device__ __forceinline__ int col(int j) const { return BKC ? tx + j * TX : (j / 4) * (4 * TX) + tx * 4 + (j & 3); }
+    __device__ __forceinline__ float value(int i, int j) const {
+        float lo, hi;
+        unpack2(acc[i][KPAIR ? j : j / 2], lo, hi);
+        return KPAIR ? lo + hi : (j & 1) ? hi : lo;
+    }
+
+    // acc += A-tile x B-tile over one BK slab
+    __device__ __forceinline__ void mma(const float *__restrict__ As, const float *__restrict__ Bs) {
+#pragma unroll
+        for (int kk = 0; kk < BK; kk += 4) {
+            if constexpr (KPAIR) {
+                ulonglong2 a2[TM], b2[TN];
+#pragma unroll
+                for (int i = 0; i < TM; ++i) a2[i] = *reinterpret_cast<const ulonglong2 *>(As + (ty + i * TY) * KP + kk);
+#pragma unroll
+                for (int j = 0; j < TN; ++j) b2[j] = *reinterpret_cast<const ulonglong2 *>(Bs + (tx + j * TX) * KP + kk);
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) {
+                        fma2(acc[i][j], a2[i].x, b2[j].x);
+                        fma2(acc[i][j], a2[i].y, b2[j].y);
+                    }
+                continue;
+            }
+            float4 a4[AKC ? TM : 1], b4[BKC ? TN : 1];
+            if constexpr (AKC) {
+#pragma unroll
+                for (int i = 0; i < TM; ++i) a4[i] = *reinterpret_cast<const float4 *>(As + (ty + i * TY) * KP + kk);
+            }
+            if constexpr (BKC) {
+#pragma unroll
+                for (int j = 0; j < TN; ++j) b4[j] = *reinterpret_cast<const float4 *>(Bs + (tx + j * TX) * KP + kk);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float a[TM];
+                unsigned long long b[TN / 2];
+                if constexpr (AKC) {
+#pragma unroll
+                    for (int i = 0; i < TM; ++i) a[i] = comp(a4[i], q);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < TM; i += 4) {
+                        const float4 v = *reinterpret_cast<const float4 *>(As + (kk + q) * (BM + 4) + (i / 4) * (4 * TY) + ty * 4);
+                        a[i] = v.x, a[i + 1] = v.y, a[i + 2] = v.z, a[i + 3] = v.w;
+                    }
+                }
+                if constexpr (BKC) {
+#pragma unroll
+                    for (int j = 0; j < TN; j += 2) b[j / 2] = pack2(comp(b4[j], q), comp(b4[j + 1], q));
+                } else {
+#pragma unroll
+                    for (int j = 0; j < TN; j += 4) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(Bs + (kk + q) * (BN + 4) + (j / 4) * (4 * TX) + tx * 4);
+                        b[j / 2] = v.x, b[j / 2 + 1] = v.y;
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < TM; ++i) {
+                    const unsigned long long aa = pack2(a[i], a[i]);
+#pragma unroll
+                    for (int j = 0; j < TN / 2; ++j) fma2(acc[i][KPAIR ? 0 : j], aa, b[j]);
+                }
+            }
+        }
+    }
+};
+
+// Fills one operand tile from a strided matrix: element (r, k) at base[r * rs + k * ks], one of the strides 1.
+// R rows of the tile start at r0 (valid below r_end), the slab starts at k0 (valid below k_end); invalid elements are zero.
+// vec: 16-byte copies are legal (base and the other stride are multiples of four elements).
+template <int R, int NT, bool KC>
+__device__ __forceinline__ void load_tile(float *dst, const float *base, long long rs, long long ks, int r0, int r_end, int k0, int k_end, bool vec,
+                                          int tid) {
+    const unsigned d = smem_u32(dst);
+    if (vec) {
+        constexpr int units = R * BK / 4;
+#pragma unroll
+        for (int u = tid; u < units; u += NT) {
+            int r, k, left;
+            unsigned at;
+            const float *src;
+            if (KC) {
+                r = u / (BK / 4);
+                k = (u % (BK / 4)) * 4;
+                at = d + (unsigned)(r * KP + k) * 4;
+                left = r0 + r < r_end ? k_end - (k0 + k) : 0;
+                src = base + (long long)(r0 + r) * rs + (k0 + k);
+            } else {
+                k = u / (R / 4);
+                r = (u % (R / 4)) * 4;
+                at = d + (unsigned)(k * (R + 4) + r) * 4;
+                left = k0 + k < k_end ? r_end - (r0 + r) : 0;
+                src = base + (long long)(k0 + k) * ks + (r0 + r);
+            }
+            const int bytes = left >= 4 ? 16 : left > 0 ? left * 4 : 0;
+            cp16(at, bytes ? src : base, bytes);
+        }
+    } else {
+        constexpr int elems = R * BK;
+#pragma unroll 4
+        for (int e = tid; e < elems; e += NT) {
+            int r, k;
+            unsigned at;
+            if (KC) {
+                r = e / BK;
+                k = e % BK;
+                at = d + (unsigned)(r * KP + k) * 4;
+            } else {
+                k = e / R;
+                r = e % R;
+                at = d + (unsigned)(k * (R + 4) + r) * 4;
+            }
+            const bool ok = r0 + r < r_end && k0 + k < k_end;
+            cp4(at, ok ? base + (long long)(r0 + r) * rs + (long long)(k0 + k) * ks : base, ok ? 4 : 0);
+        }
+    }
+}
+
+// ---- thread-block cluster along the reduction: rank and size, barrier, a peer's shared memory
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned peer_addr(unsigned addr, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ float peer_ld(unsigned addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+} // namespace simt

@@ -293,6 +293,23 @@ def test_linear_activation_f32(ops, oracle):
     close(ops.linear(x, w, b, act=2), oracle.gelu(oracle.linear(x, w, b)), 2e-5)
 
 
+# the three tiles of the f32 GEMM (32 x 32, 64 x 64, 128 x 64), their remainders, unaligned pitches, and reductions that are
+# split over the groups of a CTA and over a cluster (long k, few rows); each product is an f32 sum of k terms, added
+# in a fixed order, against the oracle's f64 sum: error of a random-sign sum of k rounded terms <= sqrt(k) * 2^-24 of its scale
+@pytest.mark.parametrize("m,k,n", [(1, 33, 31), (33, 1, 65), (31, 300, 129), (130, 2050, 10), (700, 66, 516), (2048, 100, 1030), (2, 5000, 3)])
+def test_linear_f32_tiles_and_splits(ops, m, k, n):
+    x, w, b, g = randn(m, k), randn(n, k), randn(n), randn(m, n)
+
+    def close_to(a, r, terms):
+        assert np.abs(a - r).max() <= 4.0 * np.sqrt(terms) * 2.0 ** -24 * max(1.0, np.abs(r).max())
+    x64, w64, g64 = x.astype(np.float64), w.astype(np.float64), g.astype(np.float64)
+    close_to(ops.linear(x, w, b), x64 @ w64.T + b, k)
+    dx, dw, db = ops.linear_backward(g, x, w)
+    close_to(dx, g64 @ w64, n)
+    close_to(dw, g64.T @ x64, m)
+    close_to(db, g64.sum(0), m)
+
+
 # ------------------------------------------------------------------ tensor-core GEMM
 def gemm_ref(oracle, a, a_mn, b, b_mn):
     A = oracle.round_bf16(a).astype(np.float64)
