@@ -35,6 +35,11 @@ struct mcb_ctx {
     // lazily grown scratch for reductions that need partial sums
     void *scratch = nullptr;
     size_t scratch_bytes = 0;
+    // host-to-device copies that run beside the compute stream (static steps).  d2h_async: a device-to-host copy whose end the
+    // host has not waited for may still write a host array that is copied in next: the copy stream waits for it first.
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t copy_order = nullptr;
+    bool d2h_async = false;
     // data-parallel state (owned by dp.cu)
     void *dp = nullptr;
     // optional per-kernel-class timing (mcb_prof_*): event pairs around launches
@@ -92,6 +97,8 @@ struct ProfScope {
 
 mcb_status mcb_fail(mcb_ctx *ctx, mcb_status st, const char *fmt, ...);
 mcb_status mcb_cuda_check(mcb_ctx *ctx, cudaError_t e, const char *what);
+// the copy stream, created on first use and ordered behind device-to-host copies that may still be writing host arrays
+mcb_status mcb_copy_stream(mcb_ctx *ctx, cudaStream_t *out);
 // scratch buffer of at least `bytes` (stable until a larger request)
 mcb_status mcb_scratch(mcb_ctx *ctx, size_t bytes, void **out);
 

@@ -134,6 +134,11 @@ void mcb_ctx_destroy(mcb_ctx *ctx) {
         cudaStreamDestroy(ctx->trace_stream);
     }
     if (ctx->trace_buf) cudaFree(ctx->trace_buf);
+    if (ctx->copy_stream) {
+        cudaStreamSynchronize(ctx->copy_stream);
+        cudaStreamDestroy(ctx->copy_stream);
+        cudaEventDestroy(ctx->copy_order);
+    }
     cudaFree(ctx->d_err);
     cudaFree(ctx->tc_fix_cnt);
     cudaStreamDestroy(ctx->stream);
@@ -258,6 +263,7 @@ mcb_status mcb_memcpy_d2h(mcb_ctx *ctx, void *host_dst, const void *src, size_t 
 
 mcb_status mcb_memcpy_d2h_async(mcb_ctx *ctx, void *host_dst, const void *src, size_t bytes) {
     MCB_CHECK_CTX(ctx);
+    ctx->d2h_async = true;
     if (bytes) MCB_CUDA(ctx, cudaMemcpyAsync(host_dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     return MCB_OK;
 }
@@ -390,6 +396,20 @@ mcb_status mcb_set_compute_type(mcb_ctx *ctx, int32_t compute) {
 }
 
 } // extern "C"
+
+mcb_status mcb_copy_stream(mcb_ctx *ctx, cudaStream_t *out) {
+    if (!ctx->copy_stream) {
+        MCB_CUDA(ctx, cudaEventCreateWithFlags(&ctx->copy_order, cudaEventDisableTiming));
+        MCB_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+    }
+    if (ctx->d2h_async) {
+        MCB_CUDA(ctx, cudaEventRecord(ctx->copy_order, ctx->stream));
+        MCB_CUDA(ctx, cudaStreamWaitEvent(ctx->copy_stream, ctx->copy_order, 0));
+        ctx->d2h_async = false;
+    }
+    *out = ctx->copy_stream;
+    return MCB_OK;
+}
 
 mcb_status mcb_scratch(mcb_ctx *ctx, size_t bytes, void **out) {
     if (bytes > ctx->scratch_bytes) {

@@ -27,6 +27,12 @@ struct mcb_static_step {
     int capture_id = 0;
     Tensor x, y, loss;     // fixed input buffers and the (unscaled) scalar loss
     Tensor counter;        // applied steps, when no GradScaler keeps one
+    // Inputs given as host arrays go to one of two staging buffers on the context's copy stream, beside the step that is still
+    // running, and from there to x / y on the compute stream.  taken[k]: the compute stream is done with staging buffer k.
+    Tensor stage[2];
+    size_t y_off = 0; // byte offset of y in a staging buffer
+    cudaEvent_t copied[2] = {nullptr, nullptr}, taken[2] = {nullptr, nullptr};
+    int64_t fed = 0;
     int32_t host_step_after = 0; // the host's step count as the last replay (or the creation) left it
     cudaGraphExec_t exec = nullptr;
     int64_t launches_per_step = 0;
@@ -50,6 +56,46 @@ size_t dt_size(int dt) {
     case MCB_F16: return 2;
     case MCB_BF16: return 2;
     default: return 0;
+    }
+}
+
+// x and y from the staging buffer in one launch (both areas are 16-byte aligned; the last bytes of each one by one)
+__global__ void take_inputs_kernel(const unsigned char *__restrict__ sx, unsigned char *__restrict__ x, long long nx,
+                                   const unsigned char *__restrict__ sy, unsigned char *__restrict__ y, long long ny) {
+    const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = i0; i < nx / 16; i += stride) reinterpret_cast<uint4 *>(x)[i] = reinterpret_cast<const uint4 *>(sx)[i];
+    for (long long i = i0; i < ny / 16; i += stride) reinterpret_cast<uint4 *>(y)[i] = reinterpret_cast<const uint4 *>(sy)[i];
+    if (i0 < nx % 16) x[nx / 16 * 16 + i0] = sx[nx / 16 * 16 + i0];
+    if (i0 < ny % 16) y[ny / 16 * 16 + i0] = sy[ny / 16 * 16 + i0];
+}
+
+// Copies host inputs beside the running step: PCIe needs as long for the 33.6 MB of an encoder batch as the step's
+// kernels take, and on the compute stream the two added up: 1103 us per step, side by side 615, which is PCIe alone (54 GB/s).
+mcb_status feed(mcb_static_step *s, const void *host_x, const void *host_y) {
+    mcb_ctx *ctx = s->ctx;
+    cudaStream_t cs;
+    MCB_TRY(mcb_copy_stream(ctx, &cs));
+    const int k = (int)(s->fed++ & 1);
+    const size_t nx = host_x ? dt_size(s->x.dt) * (size_t)s->x.numel() : 0, ny = host_y ? dt_size(s->y.dt) * (size_t)s->y.numel() : 0;
+    unsigned char *st = (unsigned char *)s->stage[k].ptr;
+    MCB_CUDA(ctx, cudaStreamWaitEvent(cs, s->taken[k], 0));
+    if (nx) MCB_CUDA(ctx, cudaMemcpyAsync(st, host_x, nx, cudaMemcpyHostToDevice, cs));
+    if (ny) MCB_CUDA(ctx, cudaMemcpyAsync(st + s->y_off, host_y, ny, cudaMemcpyHostToDevice, cs));
+    MCB_CUDA(ctx, cudaEventRecord(s->copied[k], cs));
+    MCB_CUDA(ctx, cudaStreamWaitEvent(ctx->stream, s->copied[k], 0));
+    take_inputs_kernel<<<mcb_grid_for(ctx, (int64_t)std::max(nx, ny) / 16 + 1, 256, 8), 256, 0, ctx->stream>>>(
+        st, (unsigned char *)s->x.ptr, (long long)nx, st + s->y_off, (unsigned char *)s->y.ptr, (long long)ny);
+    MCB_LAUNCHED(ctx);
+    MCB_CUDA(ctx, cudaEventRecord(s->taken[k], ctx->stream));
+    return MCB_OK;
+}
+
+void drop_feed(mcb_static_step *s) {
+    for (int k = 0; k < 2; ++k) {
+        if (s->copied[k]) cudaEventDestroy(s->copied[k]);
+        if (s->taken[k]) cudaEventDestroy(s->taken[k]);
+        s->copied[k] = s->taken[k] = nullptr;
+        s->stage[k] = Tensor();
     }
 }
 
@@ -161,6 +207,19 @@ mcb_status mcb_static_step_create(mcb_model *model, mcb_adam *opt, mcb_scaler *s
     MCB_TRY(new_tensor(ctx, y_dt, std::vector<int64_t>(y_dims, y_dims + y_rank), &s->y));
     MCB_TRY(mcb_memset(ctx, s->x.ptr, 0, dt_size(x_dt) * (size_t)s->x.numel()));
     MCB_TRY(mcb_memset(ctx, s->y.ptr, 0, dt_size(y_dt) * (size_t)s->y.numel()));
+    const size_t nx = dt_size(x_dt) * (size_t)s->x.numel(), ny = dt_size(y_dt) * (size_t)s->y.numel();
+    s->y_off = (nx + 255) / 256 * 256;
+    for (int k = 0; k < 2; ++k) {
+        mcb_status fs = new_tensor(ctx, MCB_U8, {(int64_t)(s->y_off + ny + 1)}, &s->stage[k]);
+        if (fs == MCB_OK) fs = mcb_cuda_check(ctx, cudaEventCreateWithFlags(&s->copied[k], cudaEventDisableTiming), "event create");
+        if (fs == MCB_OK) fs = mcb_cuda_check(ctx, cudaEventCreateWithFlags(&s->taken[k], cudaEventDisableTiming), "event create");
+        // earlier users of the block may still be enqueued on the compute stream
+        if (fs == MCB_OK) fs = mcb_cuda_check(ctx, cudaEventRecord(s->taken[k], ctx->stream), "event record");
+        if (fs != MCB_OK) {
+            drop_feed(s.get());
+            return fs;
+        }
+    }
     if (!s->scaler) {
         MCB_TRY(new_tensor(ctx, MCB_I32, {1}, &s->counter));
         // continue the bias correction where the optimizer stands (0 for a fresh one)
@@ -260,6 +319,7 @@ mcb_status mcb_static_step_create(mcb_model *model, mcb_adam *opt, mcb_scaler *s
     zero_grad(s->model->params);
     if (st != MCB_OK) {
         ctx->static_steps--;
+        drop_feed(s.get());
         s->x = Tensor();
         s->y = Tensor();
         s->loss = Tensor();
@@ -282,8 +342,7 @@ mcb_status mcb_static_step_run(mcb_static_step *s, const void *host_x, const voi
     if (!s) return MCB_INVALID_ARGUMENT;
     mcb_ctx *ctx = s->ctx;
     MCB_CHECK_CTX(ctx);
-    if (host_x) MCB_TRY(mcb_memcpy_h2d(ctx, s->x.ptr, host_x, dt_size(s->x.dt) * (size_t)s->x.numel()));
-    if (host_y) MCB_TRY(mcb_memcpy_h2d(ctx, s->y.ptr, host_y, dt_size(s->y.dt) * (size_t)s->y.numel()));
+    if (host_x || host_y) MCB_TRY(feed(s, host_x, host_y));
     if (!s->scaler) {
         // The bias correction of a step without a GradScaler reads the step's own device counter.  A checkpoint
         // load or an eager optimizer update since the last replay moved the host's count: the counter follows.
@@ -366,7 +425,9 @@ mcb_status mcb_static_step_launches(mcb_static_step *s, int64_t *kernels_per_ste
 void mcb_static_step_release(mcb_static_step *s) {
     if (!s) return;
     mcb_ctx *ctx = s->ctx;
+    if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
     cudaStreamSynchronize(ctx->stream);
+    drop_feed(s);
     if (s->exec) cudaGraphExecDestroy(s->exec);
     if (s->h_loss) cudaFreeHost(s->h_loss);
     for (int i = 0; i < 2; ++i)
