@@ -112,7 +112,7 @@ mcb_status mcb_attention(mcb_ctx *ctx, const void *q, const void *k, const void 
     // algorithmic flops: 4 N H S^2 hd forward, 10 N H S^2 hd backward (halved under a causal mask)
     ProfScope prof(ctx, MCB_PROF_ATTENTION, 4.0 * (double)n * heads * seq * seq * hd * (causal ? 0.5 : 1.0),
                    (double)total * (mcb_is_lp(dt) ? 2.0 : 4.0) * 4.0);
-    if (mcb_flash_supported(dim, heads, dt)) {
+    if (mcb_flash_supported(dim, heads, dt) && (hd == 64 || (dim % 8 == 0 && mcb_aligned16(q) && mcb_aligned16(k) && mcb_aligned16(v) && mcb_aligned16(out)))) {
         void *lse_buf = lse;
         Tmp own(ctx);
         if (!lse_buf) MCB_TRY(own.get(sizeof(float) * n * heads * seq, &lse_buf));
@@ -159,7 +159,9 @@ mcb_status mcb_attention_backward(mcb_ctx *ctx, const void *q, const void *k, co
     // algorithmic flops: 4 N H S^2 hd forward, 10 N H S^2 hd backward (halved under a causal mask)
     ProfScope prof(ctx, MCB_PROF_ATTENTION, 10.0 * (double)n * heads * seq * seq * hd * (causal ? 0.5 : 1.0),
                    (double)total * (mcb_is_lp(dt) ? 2.0 : 4.0) * 8.0);
-    if (mcb_flash_supported(dim, heads, dt) && out && lse)
+    const bool aligned = mcb_aligned16(q) && mcb_aligned16(k) && mcb_aligned16(v) && mcb_aligned16(out) && mcb_aligned16(gout) && mcb_aligned16(dq) &&
+                         mcb_aligned16(dk) && mcb_aligned16(dv);
+    if (mcb_flash_supported(dim, heads, dt) && out && lse && (hd == 64 || aligned))
         return mcb_flash_backward(ctx, q, k, v, out, gout, lse, dq, dk, dv, n, seq, dim, heads, causal, dim, dim, dim, nullptr, 0, nullptr, dt);
     float scale = 1.0f / sqrtf((float)hd);
     Tmp tmp(ctx);

@@ -1215,7 +1215,7 @@ mcb_status f_qkv_attention(const Var &x, const Var &wq, const Var &bq, const Var
     }
     const uint16_t *qp = (const uint16_t *)qkv.ptr;
     {
-        ProfScope prof(ctx, MCB_PROF_ATTENTION, 4.0 * (double)n * heads * s * s * 64 * (causal ? 0.5 : 1.0), 8.0 * (double)m * d);
+        ProfScope prof(ctx, MCB_PROF_ATTENTION, 4.0 * (double)n * d * s * s * (causal ? 0.5 : 1.0), 8.0 * (double)m * d);
         MCB_TRY(mcb_flash_forward(ctx, qp, qp + d, qp + 2 * d, o.ptr, (float *)lse.ptr, n, s, d, heads, causal, 3 * d, d, lp));
     }
     Var xv = x, wqv = wq, wkv = wk, wvv = wv, bqv = bq, bkv = bk, bvv = bv;
@@ -1228,7 +1228,7 @@ mcb_status f_qkv_attention(const Var &x, const Var &wq, const Var &bq, const Var
         uint16_t *dp = (uint16_t *)dqkv.ptr;
         const uint16_t *qp = (const uint16_t *)qkv.ptr; // the closure owns qkv, o and lse until backward has run
         {
-            ProfScope prof(ctx, MCB_PROF_ATTENTION, 10.0 * (double)n * heads * s * s * 64 * (causal ? 0.5 : 1.0), 16.0 * (double)m * d);
+            ProfScope prof(ctx, MCB_PROF_ATTENTION, 10.0 * (double)n * d * s * s * (causal ? 0.5 : 1.0), 16.0 * (double)m * d);
             // the attention backward kernels can leave per-warp column sums of dq | dk | dv (the rounded values they write): the bias
             // gradients then need only the final reduction over those rows instead of another pass over dqkv
             const int64_t brows = knob_on(ctx, K_UNFUSED_BWD) ? 0 : mcb_flash_bias_rows(n, s);

@@ -1,4 +1,6 @@
-// Fused bf16 attention for head_dim 64: forward and backward without materialising the
+// Fused 16-bit attention: the dispatcher, the delta kernel, and mma.sync kernels for bf16 with head_dim 64 (the tcgen05 kernels of
+// flash_tc.cu / flash_tc_bwd.cu serve every head dimension that is a multiple of 16 up to 128; these are kept as their
+// cross-check): forward and backward without materialising the
 // [seq, seq] probability matrix.  Online softmax in f32, products on the warp-level tensor
 // path (mma.sync m16n8k16 bf16 -> f32), operands staged in 128-byte-swizzled shared memory
 // with cp.async double buffering.
@@ -230,31 +232,31 @@ __global__ void __launch_bounds__(kThreads) flash_fwd_kernel(const bf16 *__restr
 
 // ------------------------------------------------------------------ backward: delta
 template <typename T>
-__global__ void flash_delta_kernel(const T *__restrict__ O, const T *__restrict__ dO, float *__restrict__ delta, int S, int DO, int DG, int H,
-                                   long long total_chunks) {
-    // eight lanes per (sample, row, head): 16 bytes of O and of dO each, so a warp reads 512 contiguous bytes of a row
+__global__ void flash_delta_kernel(const T *__restrict__ O, const T *__restrict__ dO, float *__restrict__ delta, int S, int DO, int DG, int H, int hd,
+                                   int lanes, long long total) {
+    // `lanes` (4, 8 or 16) lanes per (sample, row, head): 16 bytes of O and of dO each, so a warp reads consecutive bytes of a row
     dep_wait();
     dep_trigger();
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = t < total_chunks;
-    if (!live) t = total_chunks - 1;
-    const int per_row = H * (HD / 8);
-    const long long srow = t / per_row; // n * S + row
-    const int chunk = (int)(t - srow * per_row);
-    const int h = chunk >> 3;
-    const uint4 a = *reinterpret_cast<const uint4 *>(O + srow * DO + chunk * 8);
-    const uint4 b = *reinterpret_cast<const uint4 *>(dO + srow * DG + chunk * 8);
-    const uint32_t *pa = reinterpret_cast<const uint32_t *>(&a), *pb = reinterpret_cast<const uint32_t *>(&b);
+    const bool live = t < total;
+    if (!live) t = total - 1;
+    const int part = (int)(t & (lanes - 1));
+    const long long rh = t / lanes, srow = rh / H; // (n * S + row) * H + h
+    const int h = (int)(rh - srow * H);
     float v = 0.0f;
+    if (part * 8 < hd) {
+        const int col = h * hd + part * 8;
+        const uint4 a = *reinterpret_cast<const uint4 *>(O + srow * DO + col);
+        const uint4 b = *reinterpret_cast<const uint4 *>(dO + srow * DG + col);
+        const uint32_t *pa = reinterpret_cast<const uint32_t *>(&a), *pb = reinterpret_cast<const uint32_t *>(&b);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 x = Lp<T>::unpack2(pa[i]), y = Lp<T>::unpack2(pb[i]);
-        v = fmaf(x.x, y.x, fmaf(x.y, y.y, v));
+        for (int i = 0; i < 4; ++i) {
+            const float2 x = Lp<T>::unpack2(pa[i]), y = Lp<T>::unpack2(pb[i]);
+            v = fmaf(x.x, y.x, fmaf(x.y, y.y, v));
+        }
     }
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    if (live && (threadIdx.x & 7) == 0) {
+    for (int o = 1; o < lanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (live && part == 0) {
         const long long n = srow / S, row = srow - n * S;
         delta[(n * H + h) * S + row] = v;
     }
@@ -417,7 +419,11 @@ __global__ void __launch_bounds__(kThreads) flash_dkv_kernel(const bf16 *__restr
 
 } // namespace
 
-bool mcb_flash_supported(int64_t dim, int64_t heads, int32_t dt) { return mcb_is_lp(dt) && heads > 0 && dim == heads * HD; }
+bool mcb_flash_supported(int64_t dim, int64_t heads, int32_t dt) {
+    if (!mcb_is_lp(dt) || heads <= 0 || dim % heads) return false;
+    const int64_t hd = dim / heads;
+    return hd % 16 == 0 && hd > 0 && hd <= 128;
+}
 
 mcb_status mcb_flash_forward(mcb_ctx *ctx, const void *q, const void *k, const void *v, void *out, float *lse, int64_t n, int64_t seq,
                              int64_t dim, int64_t heads, int32_t causal, int64_t ldi, int64_t ldo, int32_t dt) {
@@ -426,11 +432,12 @@ mcb_status mcb_flash_forward(mcb_ctx *ctx, const void *q, const void *k, const v
         return mcb_fail(ctx, MCB_INVALID_ARGUMENT, "fused attention needs 16-byte aligned tensors");
     if (n * heads > 65535) return mcb_fail(ctx, MCB_UNSUPPORTED, "fused attention: n * heads > 65535");
     // the tcgen05 / TMEM forward first; MCB_FLASH_LEGACY (test knob) keeps the mma.sync kernel
-    if (!knob_on(ctx, K_FLASH_LEGACY) || dt == MCB_F16) {
+    const bool legacy = dt == MCB_BF16 && dim == heads * HD;
+    if (!knob_on(ctx, K_FLASH_LEGACY) || !legacy) {
         mcb_status tc = mcb_flash_tc_forward(ctx, q, k, v, out, lse, n, seq, dim, heads, causal, ldi, ldo, dt);
         if (tc != MCB_UNSUPPORTED) return tc;
     }
-    if (dt != MCB_BF16) return mcb_fail(ctx, MCB_UNSUPPORTED, "fused f16 attention: shape outside the tensor-core kernel's range");
+    if (!legacy) return mcb_fail(ctx, MCB_UNSUPPORTED, "fused attention: shape outside the tensor-core kernel's range");
     float scale_log2 = (1.0f / sqrtf((float)HD)) * 1.4426950408889634f;
     dim3 grid((unsigned)((seq + TILE - 1) / TILE), (unsigned)(n * heads));
     if (causal)
@@ -444,7 +451,6 @@ mcb_status mcb_flash_forward(mcb_ctx *ctx, const void *q, const void *k, const v
 mcb_status mcb_flash_backward(mcb_ctx *ctx, const void *q, const void *k, const void *v, const void *out, const void *gout, const float *lse,
                               void *dq, void *dk, void *dv, int64_t n, int64_t seq, int64_t dim, int64_t heads, int32_t causal,
                               int64_t ldi, int64_t ldo, int64_t ldg, float *bias_partial, int64_t bias_ld, int *bias_done, int32_t dt) {
-    (void)dim;
     if (bias_done) *bias_done = 0;
     if (ldi % 8 || ldo % 8 || ldg % 8) return mcb_fail(ctx, MCB_INVALID_ARGUMENT, "fused attention needs row pitches that are multiples of 8");
     if (n * heads > 65535) return mcb_fail(ctx, MCB_UNSUPPORTED, "fused attention: n * heads > 65535");
@@ -455,16 +461,19 @@ mcb_status mcb_flash_backward(mcb_ctx *ctx, const void *q, const void *k, const 
     void *delta = nullptr;
     MCB_TRY(mcb_alloc(ctx, sizeof(float) * rows, &delta));
     {
-        const long long chunks = rows * (HD / 8);
+        const int hd = (int)(dim / heads), lanes = hd <= 32 ? 4 : hd <= 64 ? 8 : 16;
+        const long long total = rows * lanes;
+        const dim3 dgrid((unsigned)((total + 255) / 256));
         // gout has the pitch of out; ldg is the pitch of dq / dk / dv
         if (dt == MCB_F16)
-            MCB_CUDA(ctx, mcb_launch_dep(ctx, flash_delta_kernel<__half>, dim3((unsigned)((chunks + 255) / 256)), dim3(256), 0, (const __half *)out, (const __half *)gout, (float *)delta, (int)seq, (int)ldo, (int)ldo, (int)heads, chunks));
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, flash_delta_kernel<__half>, dgrid, dim3(256), 0, (const __half *)out, (const __half *)gout, (float *)delta, (int)seq, (int)ldo, (int)ldo, (int)heads, hd, lanes, total));
         else
-            MCB_CUDA(ctx, mcb_launch_dep(ctx, flash_delta_kernel<bf16>, dim3((unsigned)((chunks + 255) / 256)), dim3(256), 0, (const bf16 *)out, (const bf16 *)gout, (float *)delta, (int)seq, (int)ldo, (int)ldo, (int)heads, chunks));
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, flash_delta_kernel<bf16>, dgrid, dim3(256), 0, (const bf16 *)out, (const bf16 *)gout, (float *)delta, (int)seq, (int)ldo, (int)ldo, (int)heads, hd, lanes, total));
     }
     ctx->launches++;
     // the tcgen05 / TMEM kernels first; MCB_FLASH_LEGACY (test knob) keeps the mma.sync pair
-    if ((!knob_on(ctx, K_FLASH_LEGACY) && !knob_on(ctx, K_FLASH_LEGACY_BWD)) || dt == MCB_F16) {
+    const bool legacy = dt == MCB_BF16 && dim == heads * HD;
+    if ((!knob_on(ctx, K_FLASH_LEGACY) && !knob_on(ctx, K_FLASH_LEGACY_BWD)) || !legacy) {
         mcb_status tc = mcb_flash_tc_backward(ctx, q, k, v, gout, lse, (const float *)delta, dq, dk, dv, n, seq, dim, heads, causal, ldi, ldo, ldg,
                                               bias_partial, bias_ld, dt);
         if (tc != MCB_UNSUPPORTED) {
@@ -473,9 +482,9 @@ mcb_status mcb_flash_backward(mcb_ctx *ctx, const void *q, const void *k, const 
             return tc;
         }
     }
-    if (dt != MCB_BF16) {
+    if (!legacy) {
         mcb_free(ctx, delta);
-        return mcb_fail(ctx, MCB_UNSUPPORTED, "fused f16 attention backward: shape outside the tensor-core kernel's range");
+        return mcb_fail(ctx, MCB_UNSUPPORTED, "fused attention backward: shape outside the tensor-core kernel's range");
     }
     dim3 grid((unsigned)((seq + TILE - 1) / TILE), (unsigned)(n * heads));
     if (causal) {

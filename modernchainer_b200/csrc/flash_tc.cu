@@ -1,4 +1,4 @@
-// Fused attention forward on the tcgen05 tensor cores (bf16, head_dim 64).
+// Fused attention forward on the tcgen05 tensor cores (bf16 / f16, head dimensions that are multiples of 16 up to 128).
 //
 // One CTA per (128-query tile, sample, head); it walks the key/value tiles of 128 keys that the
 // tile may see (all of them, or up to the diagonal when causal):
@@ -15,6 +15,11 @@
 // bf16 through shared memory and TMA, log-sum-exp per row for the backward pass).  The next S = Q K^T
 // is issued as soon as the softmax rows have read the previous S, so it overlaps the exponentials.
 // Two CTAs fit on an SM (about 97 KB of shared memory and 256 TMEM columns each).
+// Head dimension: tiles are kept as blocks of 64 columns (one 128-byte swizzled row per sequence position): one block up
+// to 64, two up to 128 (one CTA per SM then).  A head that is narrower than its blocks reads its neighbour's columns into the
+// rest of the last block: Q K^T stops after hd / 16 steps, and the columns of O past hd are never written out.  Every
+// head dimension is an instantiation of its own: the MMA sequence must be free of run-time conditions (with one, the compiler's
+// uniform registers carried a neighbouring step's operand addresses).  hd = 64 stores by TMA boxes, the others row by row.
 // Every mbarrier wait is bounded; on expiry the CTA raises the device error word and drains.
 #include "internal.h"
 #include "tc_ptx.cuh"
@@ -23,33 +28,44 @@ using namespace tcptx;
 
 namespace {
 
-constexpr int HD = 64;    // head dimension
 constexpr int BM = 128;   // queries per CTA
 constexpr int BN = 128;   // keys per tile
 constexpr int kThreads = 192;
-constexpr int kTileBytes = 128 * 64 * 2; // a [128 x 64] bf16 tile: 16 KB
+constexpr int kBlockBytes = 128 * 64 * 2; // a [128 x 64] 16-bit tile: 16 KB
 constexpr int kStages = 2;
-// shared memory: Q | K0 V0 | K1 V1 | output staging (16 KB) | barriers.  P never touches shared memory: it goes from
+// shared memory: Q | K0 V0 | K1 V1 | output staging (16 KB per block) | barriers.  P never touches shared memory: it goes from
 // the softmax registers into TMEM and is the A operand of P V from there.
-constexpr int kSmemQ = 0, kSmemKV = kTileBytes, kSmemP = kSmemKV + kStages * 2 * kTileBytes, kSmemBar = kSmemP + kTileBytes;
-// Two CTAs must fit in the SM's 228 KB (each also pays 1 KB of system reservation): 115,712 bytes at most.
-// The alignment slack is therefore 768 bytes, not 1024; the kernel checks that the aligned carve-up fits.
-constexpr int kSmemBytes = kSmemBar + 128 + 768;
-static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
-constexpr unsigned kTmemCols = 256; // S: columns [0,128), O: [128,192), P as packed bf16 pairs: [192,256)
-constexpr unsigned kColS = 0, kColO = 128, kColP = 192;
+template <int NB> struct Layout {
+    static constexpr int kTileBytes = NB * kBlockBytes;
+    static constexpr int kSmemQ = 0, kSmemKV = kTileBytes, kSmemP = kSmemKV + kStages * 2 * kTileBytes, kSmemBar = kSmemP + kTileBytes;
+    // Two CTAs must fit in the SM's 228 KB (each also pays 1 KB of system reservation): 115,712 bytes at most.
+    // The alignment slack is therefore 768 bytes, not 1024; the kernel checks that the aligned carve-up fits.
+    static constexpr int kSmemBytes = kSmemBar + 128 + 768;
+    static constexpr int kCtas = NB == 1 ? 2 : 1;
+    static_assert(kCtas * (kSmemBytes + 1024) <= 228 * 1024, "shared memory of the resident CTAs");
+    // S: columns [0,128), O: 64 per block from 128, P as packed 16-bit pairs: 64 columns behind O
+    static constexpr unsigned kTmemCols = NB == 1 ? 256 : 512;
+    static constexpr unsigned kColS = 0, kColO = 128, kColP = 128 + 64 * NB;
+};
 
 struct FwdArgs {
     float *lse;        // [n, heads, seq]
     int seq, heads, causal;
     float scale_log2;  // 1/sqrt(hd) * log2(e)
     unsigned int *err;
+    void *out;         // where the rows of a head go when its dimension is not 64
+    long long ldo;
 };
 
-template <bool F16>
-__global__ void __launch_bounds__(kThreads, 2)
+template <bool F16, int HD>
+__global__ void __launch_bounds__(kThreads, Layout<(HD > 64 ? 2 : 1)>::kCtas)
 flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_o, FwdArgs args) {
+    constexpr int NB = HD > 64 ? 2 : 1; // blocks of 64 columns
+    using L = Layout<NB>;
+    constexpr int kTileBytes = L::kTileBytes, kSmemQ = L::kSmemQ, kSmemKV = L::kSmemKV, kSmemP = L::kSmemP, kSmemBar = L::kSmemBar,
+                  kSmemBytes = L::kSmemBytes;
+    constexpr unsigned kTmemCols = L::kTmemCols, kColS = L::kColS, kColO = L::kColO, kColP = L::kColP;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char *sQ = smem + kSmemQ, *sP = smem + kSmemP;
@@ -111,7 +127,8 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // ------------------------------------------------------------ TMA producer
         if (lane == 0) {
             mbar_expect_tx(q_full, kTileBytes);
-            tma_load_3d(sQ, &map_q, q_full, h * HD, q0, n);
+            #pragma unroll
+                for (int b = 0; b < NB; ++b) tma_load_3d(sQ + b * kBlockBytes, &map_q, q_full, h * HD + b * 64, q0, n);
             bool ok = true;
             for (int j = 0; j < nt && ok; ++j) {
                 const int st = j & 1;
@@ -120,11 +137,13 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 ok = mbar_wait(&k_empty[st], ph, abort_flag, args.err);
                 if (!ok) break;
                 mbar_expect_tx(&k_full[st], kTileBytes);
-                tma_load_3d(sk, &map_k, &k_full[st], h * HD, j * BN, n);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) tma_load_3d(sk + b * kBlockBytes, &map_k, &k_full[st], h * HD + b * 64, j * BN, n);
                 ok = mbar_wait(&v_empty[st], ph, abort_flag, args.err);
                 if (!ok) break;
                 mbar_expect_tx(&v_full[st], kTileBytes);
-                tma_load_3d(sv, &map_v, &v_full[st], h * HD, j * BN, n);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) tma_load_3d(sv + b * kBlockBytes, &map_v, &v_full[st], h * HD + b * 64, j * BN, n);
             }
             // drain: every stage that was filled has been consumed before this CTA can exit
             for (int st = 0; st < kStages && ok; ++st) {
@@ -142,15 +161,17 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
             constexpr unsigned idesc_s = make_idesc(BM, BN, 0, 0, F16);   // S = Q K^T: both operands K-major
-            constexpr unsigned idesc_o = make_idesc(BM, HD, 0, 1, F16);   // O += P V: V is [keys, hd] = MN-major B
+            constexpr unsigned idesc_o = make_idesc(BM, 64 * NB, 0, 1, F16); // O += P V: V is [keys, columns] = MN-major B, whole blocks of 64
             const unsigned tmem_s = tmem_base + kColS, tmem_o = tmem_base + kColO;
             const unsigned a_q = smem_u32(sQ);
             bool ok = mbar_wait(q_full, 0, abort_flag, args.err);
             auto issue_s = [&](int j) {
                 const unsigned b_k = smem_u32(smem + kSmemKV + (j & 1) * 2 * kTileBytes);
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks)
-                    tc_mma(tmem_s, make_desc(a_q + ks * 32, 16, 1024), make_desc(b_k + ks * 32, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+                for (int ks = 0; ks < HD / 16; ++ks) {
+                    const unsigned off = (ks >> 2) * kBlockBytes + (ks & 3) * 32;
+                    tc_mma(tmem_s, make_desc(a_q + off, 16, 1024), make_desc(b_k + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+                }
                 tc_commit(s_full);
                 tc_commit(&k_empty[j & 1]);
             };
@@ -177,7 +198,7 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                 for (int ks = 0; ks < BN / 16; ++ks) {
                     // P from TMEM: 16 keys = 8 columns of packed pairs per step; V: 16 keys = 2048 bytes per step
-                    unsigned long long bd = make_desc(b_v + ks * 2048, 8192, 1024);
+                    unsigned long long bd = make_desc(b_v + ks * 2048, NB == 1 ? 8192 : kBlockBytes, 1024);
                     tc_mma_ta(tmem_o, tmem_base + kColP + ks * 8, bd, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
                 }
                 tc_commit(pv_done);
@@ -259,7 +280,7 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             if (any_move) { // warp-uniform: rows whose maximum did not move multiply by exactly 1
 #pragma unroll 1
-                for (int c = 0; c < HD / 32; ++c) {
+                for (int c = 0; c < (HD + 31) / 32; ++c) {
                     unsigned o[32];
                     tmem_ld32(tmem_base + lane_addr + kColO + c * 32, o);
                     tmem_ld_wait();
@@ -282,9 +303,9 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (ok) {
             tc_fence_after();
             const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-            unsigned char *stage = sP + wq * 4096; // this warp's [32 rows x 128 bytes] box
+            unsigned char *stage = sP + wq * (NB * 4096); // this warp's [32 rows x 128 bytes] boxes, one per block of 64 columns
 #pragma unroll 1
-            for (int c = 0; c < HD / 32; ++c) {
+            for (int c = 0; c < (HD + 31) / 32; ++c) {
                 unsigned o[32];
                 tmem_ld32(tmem_base + lane_addr + kColO + c * 32, o);
                 tmem_ld_wait();
@@ -296,12 +317,22 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     piece.z = pack16<F16>(__uint_as_float(o[q * 8 + 4]) * inv, __uint_as_float(o[q * 8 + 5]) * inv);
                     piece.w = pack16<F16>(__uint_as_float(o[q * 8 + 6]) * inv, __uint_as_float(o[q * 8 + 7]) * inv);
                     int chunk = c * 4 + q;
-                    *(uint4 *)(stage + lane * 128 + ((chunk ^ (lane & 7)) << 4)) = piece;
+                    *(uint4 *)(stage + (chunk >> 3) * 4096 + lane * 128 + (((chunk & 7) ^ (lane & 7)) << 4)) = piece;
                 }
             }
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0 && q0 + wq * 32 < args.seq) {
+            if (HD != 64) {
+                __syncwarp();
+                const int chunks = HD / 8, live = min(32, args.seq - (q0 + wq * 32));
+                uint16_t *o = (uint16_t *)args.out + ((long long)n * args.seq + q0 + wq * 32) * args.ldo + h * HD;
+                for (int i = lane; i < live * chunks; i += 32) {
+                    const int r = i / chunks, c = i - r * chunks;
+                    *(uint4 *)(o + r * args.ldo + c * 8) = *(const uint4 *)(stage + (c >> 3) * 4096 + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+                }
+            } else {
+                fence_async_smem();
+                __syncwarp();
+            }
+            if (HD == 64 && lane == 0 && q0 + wq * 32 < args.seq) {
                 tma_store_3d(&map_o, stage, h * HD, q0 + wq * 32, n);
                 bulk_commit();
                 bulk_wait_read0(); // the staging tile has been read; the write itself completes before the grid does
@@ -348,16 +379,22 @@ mcb_status make_map3(mcb_ctx *ctx, CUtensorMap *map, const void *base, long long
 
 } // namespace
 
-bool mcb_flash_tc_supported(int64_t dim, int64_t heads, int64_t ldi, int64_t ldo, const void *q, const void *k, const void *v, const void *out) {
-    return heads > 0 && dim == heads * HD && ldi % 8 == 0 && ldo % 8 == 0 && mcb_aligned16(q) && mcb_aligned16(k) && mcb_aligned16(v) &&
-           mcb_aligned16(out);
+template <int HD>
+static mcb_status launch(mcb_ctx *ctx, bool f16, dim3 grid, const CUtensorMap &mq, const CUtensorMap &mk, const CUtensorMap &mv, const CUtensorMap &mo,
+                         const FwdArgs &a) {
+    constexpr int smem = Layout<(HD > 64 ? 2 : 1)>::kSmemBytes;
+    auto kernel = f16 ? flash_tc_fwd_kernel<true, HD> : flash_tc_fwd_kernel<false, HD>;
+    MCB_CUDA(ctx, mcb_smem_limit(ctx, kernel, smem));
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, kernel, grid, dim3(kThreads), smem, mq, mk, mv, mo, a));
+    MCB_LAUNCHED(ctx);
+    return MCB_OK;
 }
 
 mcb_status mcb_flash_tc_forward(mcb_ctx *ctx, const void *q, const void *k, const void *v, void *out, float *lse, int64_t n, int64_t seq,
                                 int64_t dim, int64_t heads, int32_t causal, int64_t ldi, int64_t ldo, int32_t dt) {
-    if (!mcb_is_lp(dt)) return MCB_UNSUPPORTED;
     const bool f16 = dt == MCB_F16;
-    if (!mcb_flash_tc_supported(dim, heads, ldi, ldo, q, k, v, out)) return MCB_UNSUPPORTED;
+    if (!mcb_flash_supported(dim, heads, dt) || ldi % 8 || ldo % 8) return MCB_UNSUPPORTED;
+    if (!mcb_aligned16(q) || !mcb_aligned16(k) || !mcb_aligned16(v) || !mcb_aligned16(out)) return MCB_UNSUPPORTED;
     if (n * heads > 65535) return MCB_UNSUPPORTED;
     if (n == 0 || seq == 0) return MCB_OK;
     CUtensorMap mq, mk, mv, mo;
@@ -370,17 +407,20 @@ mcb_status mcb_flash_tc_forward(mcb_ctx *ctx, const void *q, const void *k, cons
     a.seq = (int)seq;
     a.heads = (int)heads;
     a.causal = causal;
-    a.scale_log2 = (1.0f / sqrtf((float)HD)) * 1.4426950408889634f;
+    a.scale_log2 = (1.0f / sqrtf((float)(dim / heads))) * 1.4426950408889634f;
     a.err = ctx->d_err;
-    static bool attr_set = false;
-    if (!attr_set) {
-        MCB_CUDA(ctx, cudaFuncSetAttribute(flash_tc_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        MCB_CUDA(ctx, cudaFuncSetAttribute(flash_tc_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        attr_set = true;
+    a.out = out;
+    a.ldo = ldo;
+    const dim3 grid((unsigned)((seq + BM - 1) / BM), (unsigned)(n * heads));
+    switch (dim / heads) {
+    case 16: return launch<16>(ctx, f16, grid, mq, mk, mv, mo, a);
+    case 32: return launch<32>(ctx, f16, grid, mq, mk, mv, mo, a);
+    case 48: return launch<48>(ctx, f16, grid, mq, mk, mv, mo, a);
+    case 64: return launch<64>(ctx, f16, grid, mq, mk, mv, mo, a);
+    case 80: return launch<80>(ctx, f16, grid, mq, mk, mv, mo, a);
+    case 96: return launch<96>(ctx, f16, grid, mq, mk, mv, mo, a);
+    case 112: return launch<112>(ctx, f16, grid, mq, mk, mv, mo, a);
+    case 128: return launch<128>(ctx, f16, grid, mq, mk, mv, mo, a);
+    default: return MCB_UNSUPPORTED;
     }
-    dim3 grid((unsigned)((seq + BM - 1) / BM), (unsigned)(n * heads));
-    if (f16) MCB_CUDA(ctx, mcb_launch_dep(ctx, flash_tc_fwd_kernel<true>, grid, dim3(kThreads), kSmemBytes, mq, mk, mv, mo, a));
-    else MCB_CUDA(ctx, mcb_launch_dep(ctx, flash_tc_fwd_kernel<false>, grid, dim3(kThreads), kSmemBytes, mq, mk, mv, mo, a));
-    MCB_LAUNCHED(ctx);
-    return MCB_OK;
 }

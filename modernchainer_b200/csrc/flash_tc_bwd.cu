@@ -19,6 +19,13 @@
 // delta = rowsum(O * dO) and the log-sum-exp come from the forward pass / a small pre-kernel.
 // Roles (320 threads): warp 0 TMA, warp 1 MMA + TMEM, warps 2..9 the pair arithmetic and the epilogue.
 // Every mbarrier wait is bounded; on expiry the CTA raises the device error word and drains.
+// Head dimension (multiples of 16 up to 128): tiles are blocks of 64 columns as in flash_tc.cu, one block up to 64, two up to
+// 128; S and dP stop after hd / 16 steps, the accumulators cover whole blocks and only their first hd columns are stored.
+// With two blocks the resident pair, ONE streamed stage, P and dS fill the shared memory (the next streamed pair is
+// requested once the current one's MMAs have run) and dV | dK take all of the 256 accumulator columns, so they do
+// not alternate: the rows start the next job's first pair only after they have read the accumulators, and every MMA into them
+// waits for that pair.  MODE 1 exists for hd = 64
+// only.  Each head dimension is an instantiation of its own, so that no MMA is issued under a run-time condition.
 #include "internal.h"
 #include "tc_ptx.cuh"
 
@@ -26,14 +33,18 @@ using namespace tcptx;
 
 namespace {
 
-constexpr int HD = 64;
 constexpr int BT = 128;  // tile edge: queries and keys per tile
 constexpr int kThreads = 320;
-constexpr int kTileBytes = BT * HD * 2;  // 16 KB
-// shared memory: X0 X1 (resident pair) | Y0 Y1 x 2 stages (streamed pair) | P | dS | barriers
-constexpr int kSmemX = 0, kSmemY = 2 * kTileBytes, kSmemP = kSmemY + 4 * kTileBytes, kSmemDS = kSmemP + 2 * kTileBytes,
-              kSmemBar = kSmemDS + 2 * kTileBytes;
-constexpr int kSmemBytes = kSmemBar + 128 + 1024;
+constexpr int kBlockBytes = BT * 64 * 2;  // 16 KB
+constexpr int kPairBytes = 2 * kBlockBytes; // P or dS of one pair of tiles
+// shared memory: X0 X1 (resident pair) | Y0 Y1 x stages (streamed pair) | P | dS | barriers
+template <int NB> struct Layout {
+    static constexpr int kTileBytes = NB * kBlockBytes, kStages = NB == 1 ? 2 : 1;
+    static constexpr int kSmemX = 0, kSmemY = 2 * kTileBytes, kSmemP = kSmemY + kStages * 2 * kTileBytes, kSmemDS = kSmemP + kPairBytes,
+                         kSmemBar = kSmemDS + kPairBytes;
+    static constexpr int kSmemBytes = kSmemBar + 128 + 1024;
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory of a CTA");
+};
 constexpr unsigned kTmemCols = 512;
 constexpr unsigned kColS = 0, kColDP = 128, kColAcc0 = 256, kColAcc1 = 320;
 constexpr unsigned kColDSt = 320; // MODE 1: dS as packed bf16 pairs (64 columns), the A operand of dQ += dS K, read from TMEM
@@ -52,8 +63,42 @@ struct BwdArgs {
     // MODE 0 only, optional: where to leave dS of every pair for flash_tc_dq_kernel, [sample * heads + head][query tile][key tile]
     // blocks of kDsBytes (the shared-memory tile as it is)
     unsigned char *ds_out;
+    // where rows go when the head dimension is not 64 (MODE 0: dV, dK)
+    void *out0, *out1;
+    long long ldg;
 };
-constexpr int kDsBytes = 2 * kTileBytes;
+constexpr int kDsBytes = kPairBytes;
+
+// This warp's staged boxes ([32 rows x 128 bytes] per block of 64 columns, 128-byte swizzle) as rows of a head slice: what TMA
+// does for hd = 64, by 16-byte stores where a box would reach into the next head.
+__device__ __forceinline__ void store_boxes(const unsigned char *stage, void *out, long long ld, long long first_row, int live, int col, int hd, int lane) {
+    const int chunks = hd / 8;
+    uint16_t *o = (uint16_t *)out + first_row * ld + col;
+    for (int i = lane; i < live * chunks; i += 32) {
+        const int r = i / chunks, c = i - r * chunks;
+        *(uint4 *)(o + r * ld + c * 8) = *(const uint4 *)(stage + (c >> 3) * 4096 + r * 128 + (((c & 7) ^ (r & 7)) << 4));
+    }
+}
+// column sums of the staged rows (the rounded values): lane l takes the column pairs l, l + 32
+template <bool F16> __device__ __forceinline__ void box_colsum(const unsigned char *stage, float *dst, int live, int hd, int lane) {
+    for (int cp = lane; cp < hd / 2; cp += 32) {
+        float c0 = 0.0f, c1 = 0.0f;
+        const unsigned char *box = stage + (cp >> 5) * 4096;
+        const int l = cp & 31;
+        for (int rr = 0; rr < live; ++rr) {
+            const unsigned w2 = *(const unsigned *)(box + rr * 128 + (((l >> 2) ^ (rr & 7)) << 4) + (l & 3) * 4);
+            if (F16) {
+                const float2 pr = __half22float2(*reinterpret_cast<const __half2 *>(&w2));
+                c0 += pr.x;
+                c1 += pr.y;
+            } else {
+                c0 += __uint_as_float(w2 << 16);
+                c1 += __uint_as_float(w2 & 0xFFFF0000u);
+            }
+        }
+        *(float2 *)(dst + 2 * cp) = make_float2(c0, c1);
+    }
+}
 
 // One job = one (owned tile, sample, head).  Jobs are numbered heaviest first (job / nh_total is the weight rank: under a
 // causal mask the owned tile that walks the most streamed tiles) and dealt to the persistent CTAs in boustrophedon order
@@ -83,11 +128,16 @@ template <int MODE> __device__ __forceinline__ bool job_at(const BwdArgs &args, 
 // so the next job's resident tiles are loaded as soon as the last S / dP of the current job has read the old ones, its
 // first S / dP are issued behind the current job's last accumulating MMAs, and its first pair's arithmetic follows the
 // current job's epilogue directly.  The accumulators alternate between two sets of TMEM columns from job to job.
-template <int MODE, bool F16>
+template <int MODE, bool F16, int HD>
 __global__ void __launch_bounds__(kThreads, 1)
 flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                     const __grid_constant__ CUtensorMap map_do, const __grid_constant__ CUtensorMap map_out0,
                     const __grid_constant__ CUtensorMap map_out1, BwdArgs args) {
+    constexpr int NB = HD > 64 ? 2 : 1; // blocks of 64 columns
+    using L = Layout<NB>;
+    constexpr int kTileBytes = L::kTileBytes, kSmemX = L::kSmemX, kSmemY = L::kSmemY, kSmemP = L::kSmemP, kSmemDS = L::kSmemDS, kSmemBar = L::kSmemBar;
+    constexpr unsigned ST = L::kStages; // streamed stages
+    static_assert(MODE == 0 || HD == 64, "the recomputing dQ kernel is for head dimension 64");
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char *sX0 = smem + kSmemX, *sX1 = sX0 + kTileBytes, *sP = smem + kSmemP, *sDS = smem + kSmemDS;
@@ -148,31 +198,27 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 if (it > 0) ok = mbar_wait(x_empty, (unsigned)(it - 1) & 1u, abort_flag, args.err);
                 if (!ok) break;
                 mbar_expect_tx(x_full, 2 * kTileBytes);
-                if (MODE == 0) {
-                    tma_load_3d(sX0, &map_k, x_full, jb.h * HD, jb.o0, jb.n);
-                    tma_load_3d(sX1, &map_v, x_full, jb.h * HD, jb.o0, jb.n);
-                } else {
-                    tma_load_3d(sX0, &map_q, x_full, jb.h * HD, jb.o0, jb.n);
-                    tma_load_3d(sX1, &map_do, x_full, jb.h * HD, jb.o0, jb.n);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    tma_load_3d(sX0 + b * kBlockBytes, MODE == 0 ? &map_k : &map_q, x_full, jb.h * HD + b * 64, jb.o0, jb.n);
+                    tma_load_3d(sX1 + b * kBlockBytes, MODE == 0 ? &map_v : &map_do, x_full, jb.h * HD + b * 64, jb.o0, jb.n);
                 }
                 for (int t = 0; t < jb.nt && ok; ++t, ++g) {
-                    const unsigned st = g & 1u;
-                    ok = mbar_wait(&y_empty[st], ((g >> 1) & 1u) ^ 1u, abort_flag, args.err);
+                    const unsigned st = g % ST;
+                    ok = mbar_wait(&y_empty[st], ((g / ST) & 1u) ^ 1u, abort_flag, args.err);
                     if (!ok) break;
                     unsigned char *y0 = smem + kSmemY + st * 2 * kTileBytes, *y1 = y0 + kTileBytes;
                     const int r0 = (jb.t_first + t) * BT;
                     mbar_expect_tx(&y_full[st], 2 * kTileBytes);
-                    if (MODE == 0) {
-                        tma_load_3d(y0, &map_q, &y_full[st], jb.h * HD, r0, jb.n);
-                        tma_load_3d(y1, &map_do, &y_full[st], jb.h * HD, r0, jb.n);
-                    } else {
-                        tma_load_3d(y0, &map_k, &y_full[st], jb.h * HD, r0, jb.n);
-                        tma_load_3d(y1, &map_v, &y_full[st], jb.h * HD, r0, jb.n);
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        tma_load_3d(y0 + b * kBlockBytes, MODE == 0 ? &map_q : &map_k, &y_full[st], jb.h * HD + b * 64, r0, jb.n);
+                        tma_load_3d(y1 + b * kBlockBytes, MODE == 0 ? &map_do : &map_v, &y_full[st], jb.h * HD + b * 64, r0, jb.n);
                     }
                 }
             }
-            for (unsigned st = 0; st < 2 && ok; ++st) { // drain: every stage that was filled has been consumed
-                const unsigned fills = (g > st) ? ((g - 1 - st) / 2 + 1) : 0;
+            for (unsigned st = 0; st < ST && ok; ++st) { // drain: every stage that was filled has been consumed
+                const unsigned fills = (g > st) ? ((g - 1 - st) / ST + 1) : 0;
                 if (fills) ok = mbar_wait(&y_empty[st], (fills - 1) & 1u, abort_flag, args.err);
             }
             if (*abort_flag) {
@@ -185,18 +231,22 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // ------------------------------------------------------------ MMA issuer
         if (lane == 0) {
             constexpr unsigned idesc_sd = make_idesc(BT, BT, 0, 0, F16);                       // S, dP: both operands K-major
-            constexpr unsigned idesc_acc = make_idesc(BT, HD, MODE == 0 ? 1 : 0, 1, F16);      // MODE 0: A = P^T / dS^T (MN-major); MODE 1: A = dS (K-major)
+            constexpr unsigned idesc_acc = make_idesc(BT, 64 * NB, MODE == 0 ? 1 : 0, 1, F16); // MODE 0: A = P^T / dS^T (MN-major); MODE 1: A = dS (K-major)
             const unsigned x0 = smem_u32(sX0), x1 = smem_u32(sX1), p_addr = smem_u32(sP), ds_addr = smem_u32(sDS);
             auto issue_sd = [&](unsigned gg) {
-                const unsigned y0 = smem_u32(smem + kSmemY + (gg & 1u) * 2 * kTileBytes), y1 = y0 + kTileBytes;
+                const unsigned y0 = smem_u32(smem + kSmemY + (gg % ST) * 2 * kTileBytes), y1 = y0 + kTileBytes;
                 // S = Q K^T and dP = dO V^T: MODE 0 streams (Q, dO) against resident (K, V); MODE 1 the other way round
                 const unsigned a_s = MODE == 0 ? y0 : x0, b_s = MODE == 0 ? x0 : y0, a_p = MODE == 0 ? y1 : x1, b_p = MODE == 0 ? x1 : y1;
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks)
-                    tc_mma(tmem_base + kColS, make_desc(a_s + ks * 32, 16, 1024), make_desc(b_s + ks * 32, 16, 1024), idesc_sd, ks > 0 ? 1u : 0u);
+                for (int ks = 0; ks < HD / 16; ++ks) {
+                    const unsigned off = (ks >> 2) * kBlockBytes + (ks & 3) * 32;
+                    tc_mma(tmem_base + kColS, make_desc(a_s + off, 16, 1024), make_desc(b_s + off, 16, 1024), idesc_sd, ks > 0 ? 1u : 0u);
+                }
 #pragma unroll
-                for (int ks = 0; ks < HD / 16; ++ks)
-                    tc_mma(tmem_base + kColDP, make_desc(a_p + ks * 32, 16, 1024), make_desc(b_p + ks * 32, 16, 1024), idesc_sd, ks > 0 ? 1u : 0u);
+                for (int ks = 0; ks < HD / 16; ++ks) {
+                    const unsigned off = (ks >> 2) * kBlockBytes + (ks & 3) * 32;
+                    tc_mma(tmem_base + kColDP, make_desc(a_p + off, 16, 1024), make_desc(b_p + off, 16, 1024), idesc_sd, ks > 0 ? 1u : 0u);
+                }
                 tc_commit(sd_full);
             };
             Job jb, nx;
@@ -215,18 +265,22 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int it = 0; ok && have; ++it) {
                 const bool have_next = job_at<MODE>(args, it + 1, nx);
                 // accumulators of this job: MODE 0 dV | dK, MODE 1 dQ; two sets of TMEM columns, alternating from job to job
-                const unsigned acc_a = MODE == 0 ? kColAcc0 + (unsigned)(it & 1) * 128u : ((it & 1) ? kColAccAlt1 : kColAcc0);
-                const unsigned acc_b = acc_a + 64u;
+                const unsigned acc_a = NB == 2 ? kColAcc0 : MODE == 0 ? kColAcc0 + (unsigned)(it & 1) * 128u : ((it & 1) ? kColAccAlt1 : kColAcc0);
+                const unsigned acc_b = acc_a + 64u * NB;
                 for (int t = 0; t < jb.nt && ok; ++t, ++g) {
-                    const unsigned st = g & 1u;
-                    if (t + 1 < jb.nt) {
+                    const unsigned st = g % ST;
+                    auto next_sd = [&]() {
                         // next scores of this job as soon as their streamed pair is here and the rows have read the current ones
-                        ok = mbar_wait(&y_full[(g + 1) & 1u], ((g + 1) >> 1) & 1u, abort_flag, args.err);
+                        ok = mbar_wait(&y_full[(g + 1) % ST], ((g + 1) / ST) & 1u, abort_flag, args.err);
                         if (ok) ok = mbar_wait(sd_free, g & 1u, abort_flag, args.err);
-                        if (!ok) break;
+                        if (!ok) return;
                         tc_fence_after();
                         issue_sd(g + 1);
                         if (t + 2 == jb.nt) tc_commit(x_empty);
+                    };
+                    if (ST == 2 && t + 1 < jb.nt) {
+                        next_sd();
+                        if (!ok) break;
                     }
                     ok = mbar_wait(pds_full, g & 1u, abort_flag, args.err);
                     if (!ok) break;
@@ -245,13 +299,13 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                         for (int ks = 0; ks < BT / 16; ++ks) {
                             const unsigned a_off = (ks >> 2) * 8192 + (ks & 3) * 2048;
-                            tc_mma(tmem_base + acc_a, make_desc(p_addr + a_off, 16384, 1024), make_desc(y1 + ks * 2048, 8192, 1024), idesc_acc,
+                            tc_mma(tmem_base + acc_a, make_desc(p_addr + a_off, 16384, 1024), make_desc(y1 + ks * 2048, NB == 1 ? 8192 : kBlockBytes, 1024), idesc_acc,
                                    (ks > 0) ? 1u : acc);
                         }
 #pragma unroll
                         for (int ks = 0; ks < BT / 16; ++ks) {
                             const unsigned a_off = (ks >> 2) * 8192 + (ks & 3) * 2048;
-                            tc_mma(tmem_base + acc_b, make_desc(ds_addr + a_off, 16384, 1024), make_desc(y0 + ks * 2048, 8192, 1024), idesc_acc,
+                            tc_mma(tmem_base + acc_b, make_desc(ds_addr + a_off, 16384, 1024), make_desc(y0 + ks * 2048, NB == 1 ? 8192 : kBlockBytes, 1024), idesc_acc,
                                    (ks > 0) ? 1u : acc);
                         }
                     } else {
@@ -265,11 +319,15 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     if (spill) bulk_wait_read0(); // mma_done also tells the rows that dS may be overwritten
                     tc_commit(mma_done);
                     tc_commit(&y_empty[st]);
+                    if (ST == 1 && t + 1 < jb.nt) { // the one streamed stage is refilled behind the MMAs just issued
+                        next_sd();
+                        if (!ok) break;
+                    }
                     if (t + 1 == jb.nt && have_next) {
                         // first scores of the NEXT job, queued behind this job's last accumulating MMAs: they run while the
                         // rows write this job's results out
                         ok = mbar_wait(x_full, (unsigned)(it + 1) & 1u, abort_flag, args.err);
-                        if (ok) ok = mbar_wait(&y_full[(g + 1) & 1u], ((g + 1) >> 1) & 1u, abort_flag, args.err);
+                        if (ok) ok = mbar_wait(&y_full[(g + 1) % ST], ((g + 1) / ST) & 1u, abort_flag, args.err);
                         if (ok) ok = mbar_wait(sd_free, g & 1u, abort_flag, args.err);
                         if (!ok) break;
                         tc_fence_after();
@@ -377,13 +435,13 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             if (MODE == 0 || hh == 0) {
                 tc_fence_after();
                 // MODE 0: warps with hh = 0 write dV (first accumulator), hh = 1 write dK (second, times 1/sqrt(hd)); MODE 1: dQ (scaled)
-                const unsigned acc_a = MODE == 0 ? kColAcc0 + (unsigned)(it & 1) * 128u : ((it & 1) ? kColAccAlt1 : kColAcc0);
-                const unsigned col = (MODE == 0 && hh == 1) ? acc_a + 64u : acc_a;
+                const unsigned acc_a = NB == 2 ? kColAcc0 : MODE == 0 ? kColAcc0 + (unsigned)(it & 1) * 128u : ((it & 1) ? kColAccAlt1 : kColAcc0);
+                const unsigned col = (MODE == 0 && hh == 1) ? acc_a + 64u * NB : acc_a;
                 const float f = (MODE == 0 && hh == 0) ? 1.0f : args.scale;
                 const CUtensorMap *om = (MODE == 0 && hh == 1) ? &map_out1 : &map_out0;
-                unsigned char *stage = sP + (warp - 2) * 4096; // this warp's [32 rows x 128 bytes] box (P is no longer read)
+                unsigned char *stage = sP + (warp - 2) * (NB * 4096); // this warp's [32 rows x 128 bytes] boxes (P, and with two blocks dS, are no longer read)
 #pragma unroll 1
-                for (int c = 0; c < HD / 32; ++c) {
+                for (int c = 0; c < (HD + 31) / 32; ++c) {
                     unsigned o[32];
                     tmem_ld32(tmem_base + lane_addr + col + c * 32, o);
                     tmem_ld_wait();
@@ -395,30 +453,20 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         piece.z = pack16<F16>(__uint_as_float(o[q * 8 + 4]) * f, __uint_as_float(o[q * 8 + 5]) * f);
                         piece.w = pack16<F16>(__uint_as_float(o[q * 8 + 6]) * f, __uint_as_float(o[q * 8 + 7]) * f);
                         int chunk = c * 4 + q;
-                        *(uint4 *)(stage + lane * 128 + ((chunk ^ (lane & 7)) << 4)) = piece;
+                        *(uint4 *)(stage + (chunk >> 3) * 4096 + lane * 128 + (((chunk & 7) ^ (lane & 7)) << 4)) = piece;
                     }
                 }
                 fence_async_smem();
                 __syncwarp();
                 if (args.bias_partial) {
-                    // lane l sums columns 2l, 2l+1 of this warp's 32 staged rows (the rounded values; rows past the sequence end excluded)
-                    float c0 = 0.0f, c1 = 0.0f;
-                    const int rows_live = min(32, args.seq - (o0 + wq * 32));
-                    for (int rr = 0; rr < rows_live; ++rr) {
-                        const unsigned w2 = *(const unsigned *)(stage + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
-                        if (F16) {
-                            const float2 pr = __half22float2(*reinterpret_cast<const __half2 *>(&w2));
-                            c0 += pr.x;
-                            c1 += pr.y;
-                        } else {
-                            c0 += __uint_as_float(w2 << 16);
-                            c1 += __uint_as_float(w2 & 0xFFFF0000u);
-                        }
-                    }
                     const int which = MODE == 1 ? 0 : (hh == 1 ? 1 : 2); // dq, dk, dv column block of the packed gradient
-                    float *dst = args.bias_partial + ((size_t)(n * tiles + own) * 4 + wq) * args.bias_ld + which * args.dim + h * HD + 2 * lane;
-                    *(float2 *)dst = make_float2(c0, c1);
+                    box_colsum<F16>(stage, args.bias_partial + ((size_t)(n * tiles + own) * 4 + wq) * args.bias_ld + which * args.dim + h * HD,
+                                    min(32, args.seq - (o0 + wq * 32)), HD, lane);
                 }
+                if (HD != 64) {
+                    store_boxes(stage, (MODE == 0 && hh == 1) ? args.out1 : args.out0, args.ldg, (long long)n * args.seq + o0 + wq * 32,
+                                min(32, args.seq - (o0 + wq * 32)), h * HD, HD, lane);
+                } else
                 if (lane == 0 && o0 + wq * 32 < args.seq) {
                     tma_store_3d(om, stage, h * HD, o0 + wq * 32, n);
                     bulk_commit();
@@ -445,10 +493,13 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 // warps 2..5 the epilogue (scale, round, TMA store, column sums for the q bias gradient).  Every wait is bounded.
 constexpr int kDqThreads = 192;
 constexpr int kDqStages = 2;
-constexpr int kDqStageBytes = kDsBytes + kTileBytes; // 48 KB
-constexpr int kDqSmemOut = kDqStages * kDqStageBytes, kDqSmemBar = kDqSmemOut + 4 * 4096;
-constexpr int kDqSmemBytes = kDqSmemBar + 128 + 768;
-static_assert(2 * (kDqSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
+template <int NB> struct DqLayout {
+    static constexpr int kStageBytes = kDsBytes + NB * kBlockBytes; // 48 or 64 KB
+    static constexpr int kSmemOut = kDqStages * kStageBytes, kSmemBar = kSmemOut + 4 * 4096 * NB;
+    static constexpr int kSmemBytes = kSmemBar + 128 + 768;
+    static constexpr int kCtas = NB == 1 ? 2 : 1;
+    static_assert(kCtas * (kSmemBytes + 1024) <= 228 * 1024, "resident CTAs per SM");
+};
 
 struct DqArgs {
     const unsigned char *ds;
@@ -457,11 +508,17 @@ struct DqArgs {
     unsigned int *err;
     float *bias_partial;
     int bias_ld, dim;
+    int hd; // head dimension, and where rows go when it is not 64
+    void *out;
+    long long ldg;
 };
 
-template <bool F16>
-__global__ void __launch_bounds__(kDqThreads, 2)
+template <bool F16, int NB, int HDT>
+__global__ void __launch_bounds__(kDqThreads, DqLayout<NB>::kCtas)
 flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_dq, DqArgs args) {
+    using L = DqLayout<NB>;
+    constexpr int kDqStageBytes = L::kStageBytes, kDqSmemOut = L::kSmemOut, kDqSmemBar = L::kSmemBar, kDqSmemBytes = L::kSmemBytes;
+    const int HD = HDT ? HDT : args.hd;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned long long *bars = (unsigned long long *)(smem + kDqSmemBar);
@@ -491,7 +548,7 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, 64);
+        tmem_alloc(tmem_slot, 64 * NB);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -512,7 +569,8 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 unsigned char *sd = smem + st * kDqStageBytes;
                 mbar_expect_tx(&full[st], kDqStageBytes);
                 bulk_load(sd, src + (size_t)t * kDsBytes, kDsBytes, &full[st]);
-                tma_load_3d(sd + kDsBytes, &map_k, &full[st], h * HD, t * BT, n);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) tma_load_3d(sd + kDsBytes + b * kBlockBytes, &map_k, &full[st], h * HD + b * 64, t * BT, n);
             }
             for (int st = 0; st < kDqStages && ok; ++st) { // drain: nothing is still landing in shared memory at exit
                 const int fills = (nt > st) ? ((nt - 1 - st) / kDqStages + 1) : 0;
@@ -526,7 +584,7 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr unsigned idesc = make_idesc(BT, HD, 0, 1, F16); // A = dS (K-major), B = K as loaded ([keys, hd]: MN-major)
+            constexpr unsigned idesc = make_idesc(BT, 64 * NB, 0, 1, F16); // A = dS (K-major), B = K as loaded ([keys, hd]: MN-major)
             bool ok = true;
             for (int t = 0; t < nt && ok; ++t) {
                 const int st = t % kDqStages;
@@ -536,7 +594,7 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                 const unsigned ds_addr = smem_u32(smem + st * kDqStageBytes), k_addr = ds_addr + kDsBytes;
 #pragma unroll
                 for (int ks = 0; ks < BT / 16; ++ks) // 16 keys per step: 32 bytes inside a 64-key block of 16 KB
-                    tc_mma(tmem_base, make_desc(ds_addr + (ks >> 2) * 16384 + (ks & 3) * 32, 16, 1024), make_desc(k_addr + ks * 2048, 8192, 1024), idesc,
+                    tc_mma(tmem_base, make_desc(ds_addr + (ks >> 2) * 16384 + (ks & 3) * 32, 16, 1024), make_desc(k_addr + ks * 2048, NB == 1 ? 8192 : kBlockBytes, 1024), idesc,
                            (t > 0 || ks > 0) ? 1u : 0u);
                 tc_commit(&empty[st]);
             }
@@ -548,9 +606,9 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
         bool ok = nt > 0 ? mbar_wait(acc_done, 0, abort_flag, args.err) : true;
         if (ok) {
             tc_fence_after();
-            unsigned char *stage = smem + kDqSmemOut + wq * 4096; // this warp's [32 rows x 128 bytes] box
+            unsigned char *stage = smem + kDqSmemOut + wq * (NB * 4096); // this warp's [32 rows x 128 bytes] boxes
 #pragma unroll 1
-            for (int c = 0; c < HD / 32; ++c) {
+            for (int c = 0; c < (HD + 31) / 32; ++c) {
                 unsigned o[32];
                 if (nt > 0) {
                     tmem_ld32(tmem_base + lane_addr + c * 32, o);
@@ -567,28 +625,17 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
                     piece.z = pack16<F16>(__uint_as_float(o[q * 8 + 4]) * args.scale, __uint_as_float(o[q * 8 + 5]) * args.scale);
                     piece.w = pack16<F16>(__uint_as_float(o[q * 8 + 6]) * args.scale, __uint_as_float(o[q * 8 + 7]) * args.scale);
                     const int chunk = c * 4 + q;
-                    *(uint4 *)(stage + lane * 128 + ((chunk ^ (lane & 7)) << 4)) = piece;
+                    *(uint4 *)(stage + (chunk >> 3) * 4096 + lane * 128 + (((chunk & 7) ^ (lane & 7)) << 4)) = piece;
                 }
             }
             fence_async_smem();
             __syncwarp();
-            if (args.bias_partial) { // lane l sums columns 2l, 2l+1 of this warp's 32 staged rows (the rounded values)
-                float c0 = 0.0f, c1 = 0.0f;
-                const int rows_live = min(32, args.seq - (o0 + wq * 32));
-                for (int rr = 0; rr < rows_live; ++rr) {
-                    const unsigned w2 = *(const unsigned *)(stage + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
-                    if (F16) {
-                        const float2 pr = __half22float2(*reinterpret_cast<const __half2 *>(&w2));
-                        c0 += pr.x;
-                        c1 += pr.y;
-                    } else {
-                        c0 += __uint_as_float(w2 << 16);
-                        c1 += __uint_as_float(w2 & 0xFFFF0000u);
-                    }
-                }
-                float *dst = args.bias_partial + ((size_t)(n * tiles + own) * 4 + wq) * args.bias_ld + h * HD + 2 * lane;
-                *(float2 *)dst = make_float2(c0, c1);
-            }
+            if (args.bias_partial)
+                box_colsum<F16>(stage, args.bias_partial + ((size_t)(n * tiles + own) * 4 + wq) * args.bias_ld + h * HD, min(32, args.seq - (o0 + wq * 32)), HD,
+                                lane);
+            if (HDT != 64) {
+                store_boxes(stage, args.out, args.ldg, (long long)n * args.seq + o0 + wq * 32, min(32, args.seq - (o0 + wq * 32)), h * HD, HD, lane);
+            } else
             if (lane == 0 && o0 + wq * 32 < args.seq) {
                 tma_store_3d(&map_dq, stage, h * HD, o0 + wq * 32, n);
                 bulk_commit();
@@ -598,7 +645,7 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, 64);
+    if (warp == 1) tmem_dealloc(tmem_base, 64 * NB);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
@@ -640,7 +687,7 @@ mcb_status mcb_flash_tc_backward(mcb_ctx *ctx, const void *q, const void *k, con
                                  int64_t ldo, int64_t ldg, float *bias_partial, int64_t bias_ld, int32_t dt) {
     if (!mcb_is_lp(dt)) return MCB_UNSUPPORTED;
     const bool f16 = dt == MCB_F16;
-    if (heads <= 0 || dim != heads * HD || ldi % 8 || ldo % 8 || ldg % 8 || n * heads > 65535) return MCB_UNSUPPORTED;
+    if (!mcb_flash_supported(dim, heads, dt) || ldi % 8 || ldo % 8 || ldg % 8 || n * heads > 65535) return MCB_UNSUPPORTED;
     if (!mcb_aligned16(q) || !mcb_aligned16(k) || !mcb_aligned16(v) || !mcb_aligned16(gout) || !mcb_aligned16(dq) || !mcb_aligned16(dk) ||
         !mcb_aligned16(dv))
         return MCB_UNSUPPORTED;
@@ -662,7 +709,11 @@ mcb_status mcb_flash_tc_backward(mcb_ctx *ctx, const void *q, const void *k, con
     a.tiles = (int)((seq + BT - 1) / BT);
     a.nh_total = (int)(n * heads);
     a.jobs = a.tiles * a.nh_total;
-    a.scale = 1.0f / sqrtf((float)HD);
+    const int hd = (int)(dim / heads);
+    a.out0 = dv;
+    a.out1 = dk;
+    a.ldg = ldg;
+    a.scale = 1.0f / sqrtf((float)hd);
     a.scale_log2 = a.scale * 1.4426950408889634f;
     a.err = ctx->d_err;
     a.bias_partial = bias_partial;
@@ -673,45 +724,56 @@ mcb_status mcb_flash_tc_backward(mcb_ctx *ctx, const void *q, const void *k, con
     const long long tiles = (seq + BT - 1) / BT;
     const size_t ds_bytes = (size_t)n * heads * tiles * tiles * kDsBytes;
     void *ds = nullptr;
-    if (!knob_on(ctx, K_FLASH_DQ_RECOMPUTE) && ds_bytes <= ((size_t)1 << 30)) {
+    // (head dimensions other than 64 have no recomputing kernel)
+    if (hd != 64 || (!knob_on(ctx, K_FLASH_DQ_RECOMPUTE) && ds_bytes <= ((size_t)1 << 30))) {
         MCB_TRY(mcb_alloc(ctx, ds_bytes, &ds));
         a.ds_out = (unsigned char *)ds;
-    }
-    static bool attr_set = false;
-    if (!attr_set) {
-        MCB_CUDA(ctx, cudaFuncSetAttribute(flash_tc_bwd_kernel<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        MCB_CUDA(ctx, cudaFuncSetAttribute(flash_tc_bwd_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        MCB_CUDA(ctx, cudaFuncSetAttribute(flash_tc_bwd_kernel<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        MCB_CUDA(ctx, cudaFuncSetAttribute(flash_tc_bwd_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        MCB_CUDA(ctx, cudaFuncSetAttribute(flash_tc_dq_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmemBytes));
-        MCB_CUDA(ctx, cudaFuncSetAttribute(flash_tc_dq_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmemBytes));
-        attr_set = true;
     }
     const dim3 grid((unsigned)tiles, (unsigned)(n * heads));              // one CTA per job (the dQ-from-dS kernel)
     // persistent CTAs for the tile-pair kernels; MCB_FLASH_BWD_ONE_JOB (test knob) gives every job a CTA of its own
     const dim3 pgrid((unsigned)((a.jobs < ctx->sm_count || knob_on(ctx, K_FLASH_BWD_ONE_JOB)) ? a.jobs : ctx->sm_count));
-    cudaError_t e;
-    if (f16) e = mcb_launch_dep(ctx, flash_tc_bwd_kernel<0, true>, pgrid, dim3(kThreads), kSmemBytes, mq, mk, mv, mdo, mdv, mdk, a);
-    else e = mcb_launch_dep(ctx, flash_tc_bwd_kernel<0, false>, pgrid, dim3(kThreads), kSmemBytes, mq, mk, mv, mdo, mdv, mdk, a);
+    DqArgs d;
+    d.ds = (const unsigned char *)ds;
+    d.seq = (int)seq;
+    d.heads = (int)heads;
+    d.causal = causal;
+    d.scale = a.scale;
+    d.err = ctx->d_err;
+    d.bias_partial = bias_partial;
+    d.bias_ld = (int)bias_ld;
+    d.dim = (int)dim;
+    d.hd = hd;
+    d.out = dq;
+    d.ldg = ldg;
+    auto pairs = [&](auto kernel, int smem, const CUtensorMap &out0, const CUtensorMap &out1) -> cudaError_t {
+        cudaError_t e = mcb_smem_limit(ctx, kernel, smem);
+        if (e == cudaSuccess) e = mcb_launch_dep(ctx, kernel, pgrid, dim3(kThreads), smem, mq, mk, mv, mdo, out0, out1, a);
+        return e;
+    };
+    constexpr int kSmem1 = Layout<1>::kSmemBytes, kSmem2 = Layout<2>::kSmemBytes, kDq1 = DqLayout<1>::kSmemBytes, kDq2 = DqLayout<2>::kSmemBytes;
+    auto from_ds = [&](auto kernel, int smem) -> cudaError_t {
+        cudaError_t e = mcb_smem_limit(ctx, kernel, smem);
+        if (e == cudaSuccess) e = mcb_launch_dep(ctx, kernel, grid, dim3(kDqThreads), smem, mk, mdq, d);
+        return e;
+    };
+    auto dkdv = [&](auto f16_kernel, auto bf16_kernel, int smem) { return f16 ? pairs(f16_kernel, smem, mdv, mdk) : pairs(bf16_kernel, smem, mdv, mdk); };
+    cudaError_t e = cudaErrorInvalidValue;
+    switch (hd) {
+    case 16: e = dkdv(flash_tc_bwd_kernel<0, true, 16>, flash_tc_bwd_kernel<0, false, 16>, kSmem1); break;
+    case 32: e = dkdv(flash_tc_bwd_kernel<0, true, 32>, flash_tc_bwd_kernel<0, false, 32>, kSmem1); break;
+    case 48: e = dkdv(flash_tc_bwd_kernel<0, true, 48>, flash_tc_bwd_kernel<0, false, 48>, kSmem1); break;
+    case 64: e = dkdv(flash_tc_bwd_kernel<0, true, 64>, flash_tc_bwd_kernel<0, false, 64>, kSmem1); break;
+    case 80: e = dkdv(flash_tc_bwd_kernel<0, true, 80>, flash_tc_bwd_kernel<0, false, 80>, kSmem2); break;
+    case 96: e = dkdv(flash_tc_bwd_kernel<0, true, 96>, flash_tc_bwd_kernel<0, false, 96>, kSmem2); break;
+    case 112: e = dkdv(flash_tc_bwd_kernel<0, true, 112>, flash_tc_bwd_kernel<0, false, 112>, kSmem2); break;
+    case 128: e = dkdv(flash_tc_bwd_kernel<0, true, 128>, flash_tc_bwd_kernel<0, false, 128>, kSmem2); break;
+    }
     if (e == cudaSuccess) {
         ctx->launches++;
-        if (ds) {
-            DqArgs d;
-            d.ds = (const unsigned char *)ds;
-            d.seq = (int)seq;
-            d.heads = (int)heads;
-            d.causal = causal;
-            d.scale = a.scale;
-            d.err = ctx->d_err;
-            d.bias_partial = bias_partial;
-            d.bias_ld = (int)bias_ld;
-            d.dim = (int)dim;
-            if (f16) e = mcb_launch_dep(ctx, flash_tc_dq_kernel<true>, grid, dim3(kDqThreads), kDqSmemBytes, mk, mdq, d);
-            else e = mcb_launch_dep(ctx, flash_tc_dq_kernel<false>, grid, dim3(kDqThreads), kDqSmemBytes, mk, mdq, d);
-        } else {
-            if (f16) e = mcb_launch_dep(ctx, flash_tc_bwd_kernel<1, true>, pgrid, dim3(kThreads), kSmemBytes, mq, mk, mv, mdo, mdq, mdq, a);
-            else e = mcb_launch_dep(ctx, flash_tc_bwd_kernel<1, false>, pgrid, dim3(kThreads), kSmemBytes, mq, mk, mv, mdo, mdq, mdq, a);
-        }
+        if (!ds) e = f16 ? pairs(flash_tc_bwd_kernel<1, true, 64>, kSmem1, mdq, mdq) : pairs(flash_tc_bwd_kernel<1, false, 64>, kSmem1, mdq, mdq);
+        else if (hd == 64) e = f16 ? from_ds(flash_tc_dq_kernel<true, 1, 64>, kDq1) : from_ds(flash_tc_dq_kernel<false, 1, 64>, kDq1);
+        else if (hd < 64) e = f16 ? from_ds(flash_tc_dq_kernel<true, 1, 0>, kDq1) : from_ds(flash_tc_dq_kernel<false, 1, 0>, kDq1);
+        else e = f16 ? from_ds(flash_tc_dq_kernel<true, 2, 0>, kDq2) : from_ds(flash_tc_dq_kernel<false, 2, 0>, kDq2);
     }
     if (ds) mcb_free(ctx, ds); // stream-ordered reuse: whoever gets the block next is enqueued behind the dQ kernel
     MCB_CUDA(ctx, e);

@@ -56,7 +56,7 @@ mcb_status mcb_tc_gemm(mcb_ctx *ctx, const TcGemmParams &p);
 void mcb_tc_plan(mcb_ctx *ctx, int64_t m, int64_t n, int64_t k, bool allow_split, bool atomic_out, int fixed_split, int *bn_out,
                  int *split_out);
 
-// flash_attn.cu: fused bf16 attention, head_dim 64
+// flash_attn.cu: fused 16-bit attention, head dimensions that are multiples of 16 up to 128
 bool mcb_flash_supported(int64_t dim, int64_t heads, int32_t dt);
 mcb_status mcb_flash_forward(mcb_ctx *ctx, const void *q, const void *k, const void *v, void *out, float *lse, int64_t n, int64_t seq,
                              int64_t dim, int64_t heads, int32_t causal, int64_t ldi, int64_t ldo, int32_t dt = MCB_BF16);

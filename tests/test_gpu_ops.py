@@ -412,6 +412,24 @@ def test_fused_attention_bf16_head_dim_64(ops, oracle, n, s, h, causal):
         assert np.abs(a - r).max() <= max(np.abs(r).max(), 1e-3) * 2.0 ** -6, np.abs(a - r).max() / np.abs(r).max()
 
 
+# every number of 16-wide steps, one block of 64 columns and two, ragged and single-row sequences, several jobs per CTA (the
+# last three).  Bounds as for head dimension 64: the 16-bit rounding of P and dS, 2^-8 (2^-11) per product, under a
+# max-norm over the tensor
+@pytest.mark.parametrize("dt", ["bf16", "f16"])
+@pytest.mark.parametrize("n,s,h,hd,causal", [(1, 100, 2, 16, True), (2, 256, 3, 32, False), (1, 1, 1, 32, True), (2, 130, 2, 48, True),
+                                             (1, 300, 3, 80, True), (2, 129, 1, 96, False), (1, 257, 2, 112, True), (1, 128, 1, 128, False),
+                                             (40, 130, 5, 32, True), (40, 130, 5, 80, True), (20, 260, 4, 128, False)])
+def test_fused_attention_head_dims(ops, oracle, n, s, h, hd, causal, dt):
+    code, eps = (5, 2.0 ** -8) if dt == "bf16" else (4, 2.0 ** -11)
+    rounded = oracle.round_bf16 if dt == "bf16" else (lambda a: a.astype(np.float16).astype(np.float32))
+    q, k, v, g = (rounded(randn(n, s, h * hd)) for _ in range(4))
+    out, _ = ops.attention(q, k, v, h, causal, dt=code)
+    ref = oracle.attention(q, k, v, h, causal)
+    assert np.abs(out - ref).max() <= max(np.abs(ref).max(), 1e-3) * 2 * eps
+    for a, r in zip(ops.attention_backward(q, k, v, g, h, causal, dt=code), oracle.attention_backward(q, k, v, g, h, causal)):
+        assert np.abs(a - r).max() <= max(np.abs(r).max(), 1e-3) * 4 * eps, np.abs(a - r).max() / np.abs(r).max()
+
+
 @pytest.mark.parametrize("dt", ["bf16", "f16"])
 @pytest.mark.parametrize("n,s,h,causal", [(1, 64, 1, True), (2, 256, 3, True), (2, 256, 3, False), (1, 100, 2, True), (3, 130, 1, False),
                                           (1, 1024, 2, True), (2, 700, 2, True), (4, 1024, 5, True), (5, 640, 6, False)])
