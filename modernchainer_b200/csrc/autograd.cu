@@ -580,7 +580,10 @@ static int lowp_dtype(mcb_ctx *ctx) {
     if (ctx->compute == MCB_COMPUTE_F16) return MCB_F16;
     return -1;
 }
-static bool tc_shape_ok(int64_t m, int64_t n, int64_t k) { return m > 0 && (n % 8 == 0) && (k % 8 == 0) && n > 0 && k > 0; }
+// rows of the operands must be 16-byte pitched: the reduction length decides; an output width that is no multiple of 8 gets a
+// padded pitch (pad8)
+static bool tc_shape_ok(int64_t m, int64_t n, int64_t k) { return m > 0 && (k % 8 == 0) && n > 0 && k > 0; }
+static int64_t pad8(int64_t n) { return (n + 7) / 8 * 8; }
 
 // 16-bit operand (type lp) for `v`: the arena's shadow copy for parameters, the tensor itself when it
 // already has that type, otherwise a converted copy
@@ -668,6 +671,20 @@ static mcb_status linear_backward_impl(mcb_ctx *ctx, const Tensor &g_in, const L
         g = gp;
     }
     if (sv.bf16) {
+        int64_t gld = g.ld ? g.ld : n; // row pitch of the gradient as a GEMM operand
+        if (gld % 8) {
+            Tensor gp;
+            MCB_TRY(new_tensor(ctx, sv.lp, {m, pad8(n)}, &gp));
+            MCB_TRY(mcb_repitch16(ctx, g.ptr, n, gp.ptr, pad8(n), m, n));
+            if (want_db && !db_done) {
+                bool direct;
+                MCB_TRY(grad_dst(b, &gi[2], &direct));
+                MCB_TRY(mcb_col_sum(ctx, g.ptr, gdt, m, n, (float *)gi[2].ptr));
+                db_done = true;
+            }
+            g = gp;
+            gld = pad8(n);
+        }
         // The weight gradient first in the books: where it goes and whether its reduction is split.  A split one adds its
         // slices into an output that must be zero: the data-gradient GEMM in front of it clears that buffer on the side
         // (its epilogue warps are idle until the first tile is done), which saves a fill of its own per Linear.
@@ -677,7 +694,7 @@ static mcb_status linear_backward_impl(mcb_ctx *ctx, const Tensor &g_in, const L
             bool direct;
             MCB_TRY(grad_dst(w, &gi[1], &direct));
             pw.in_dt = sv.lp;
-            pw.a = g.ptr; pw.a_mn_major = 1; pw.lda = n;
+            pw.a = g.ptr; pw.a_mn_major = 1; pw.lda = gld;
             pw.b = sv.x.ptr; pw.b_mn_major = 1; pw.ldb = k;
             pw.d = gi[1].ptr; pw.out_dt = MCB_F32; pw.ldd = k;
             pw.m = n; pw.n = k; pw.k = m;
@@ -694,7 +711,7 @@ static mcb_status linear_backward_impl(mcb_ctx *ctx, const Tensor &g_in, const L
             MCB_TRY(new_tensor(ctx, xdt, x->data.shape, &gi[0]));
             TcGemmParams p; // dx[m,k] = g[m,n] * W[n,k]
             p.in_dt = sv.lp;
-            p.a = g.ptr; p.a_mn_major = 0; p.lda = n;
+            p.a = g.ptr; p.a_mn_major = 0; p.lda = gld;
             p.b = wb.ptr; p.b_mn_major = 1; p.ldb = k;
             p.d = gi[0].ptr; p.out_dt = xdt; p.ldd = k;
             p.m = m; p.n = k; p.k = n;
@@ -750,7 +767,8 @@ static mcb_status linear_backward_impl(mcb_ctx *ctx, const Tensor &g_in, const L
     return MCB_OK;
 }
 
-static mcb_status f_linear_impl(const Var &x, const Var &w, const Var &b, int act, Var *out) {
+// keep_pitch: the result of a 16-bit product whose width is no multiple of 8 keeps its padded rows (Tensor::ld)
+static mcb_status f_linear_impl(const Var &x, const Var &w, const Var &b, int act, Var *out, bool keep_pitch = false) {
     MCB_TRY(check_same_ctx(x, w));
     mcb_ctx *ctx = x->ctx;
     if (w->data.shape.size() != 2 || x->data.shape.empty() || x->data.shape.back() != w->data.shape[1])
@@ -772,22 +790,39 @@ static mcb_status f_linear_impl(const Var &x, const Var &w, const Var &b, int ac
         Tensor wb;
         MCB_TRY(to_dtype(ctx, x->data, lp, &sv->x));
         MCB_TRY(lowp_of(w, lp, &wb));
-        MCB_TRY(new_tensor(ctx, lp, oshape, &res));
+        const int64_t ldn = pad8(n);
+        auto pitched = [&](Tensor *t) -> mcb_status { // [m, n] at pitch ldn
+            MCB_TRY(new_tensor(ctx, lp, {m, ldn}, t));
+            t->shape = oshape;
+            t->ld = ldn == n ? 0 : ldn;
+            return MCB_OK;
+        };
+        auto contiguous = [&](Tensor *t) -> mcb_status {
+            if (!t->ld) return MCB_OK;
+            Tensor c;
+            MCB_TRY(new_tensor(ctx, lp, oshape, &c));
+            MCB_TRY(mcb_repitch16(ctx, t->ptr, t->ld, c.ptr, n, m, n));
+            *t = c;
+            return MCB_OK;
+        };
+        MCB_TRY(pitched(&res));
         TcGemmParams p; // y[m,n] = x[m,k] * W[n,k]^T + bias
         p.in_dt = lp;
         p.a = sv->x.ptr; p.lda = k;
         p.b = wb.ptr; p.ldb = k;
-        p.d = res.ptr; p.out_dt = lp; p.ldd = n;
+        p.d = res.ptr; p.out_dt = lp; p.ldd = ldn;
         p.bias = b ? (const float *)b->data.ptr : nullptr;
         p.m = m; p.n = n; p.k = k;
         p.act = act;
         if (act != MCB_ACT_NONE && g_grad_enabled) {
-            MCB_TRY(new_tensor(ctx, lp, oshape, &sv->pre));
+            MCB_TRY(pitched(&sv->pre));
             p.d_pre = sv->pre.ptr;
         }
         MCB_TRY(mcb_tc_gemm(ctx, p));
+        if (!keep_pitch) MCB_TRY(contiguous(&res));
+        if (sv->pre.defined) MCB_TRY(contiguous(&sv->pre));
     } else {
-        // Shapes the tensor-core kernel declines (an extent that is not a multiple of 8) keep the lowering's
+        // Shapes the tensor-core kernel declines (a reduction length that is not a multiple of 8) keep the lowering's
         // numerics under autocast: operands rounded to the 16-bit type, exact f32 products and sums, f32 result
         // (the reference lowers every linear under autocast, cuda/src/ops.rs:762-781).
         Tensor wf = w->data;
@@ -1046,11 +1081,11 @@ mcb_status f_sce_consuming(const Var &logits, const Var &target, Var *out) {
     MCB_TRY(new_tensor(ctx, MCB_F32, {}, &res));
     Tensor x = logits->data, lab = target->data, stats;
     MCB_TRY(new_tensor(ctx, MCB_F32, {n, 2}, &stats)); // row maximum and sum of exp: the gradient pass streams the rows without reducing them again
-    MCB_TRY(mcb_sce_grad(ctx, x.ptr, nullptr, x.dt, lab.ptr, ldt, n, c, (float *)res.ptr, nullptr, (float *)stats.ptr, nullptr)); // loss only
+    MCB_TRY(mcb_sce_grad(ctx, x.ptr, nullptr, x.dt, lab.ptr, ldt, n, c, (float *)res.ptr, nullptr, (float *)stats.ptr, nullptr, x.ld)); // loss only
     *out = apply(ctx, "SoftmaxCrossEntropy", res, {logits, target}, [ctx, x, lab, stats, ldt, n, c](const Tensor &g, std::vector<Tensor> &gi) -> mcb_status {
         Tensor gf;
         MCB_TRY(to_dtype(ctx, g, MCB_F32, &gf));
-        MCB_TRY(mcb_sce_grad(ctx, x.ptr, x.ptr, x.dt, lab.ptr, ldt, n, c, nullptr, (const float *)gf.ptr, nullptr, (const float *)stats.ptr));
+        MCB_TRY(mcb_sce_grad(ctx, x.ptr, x.ptr, x.dt, lab.ptr, ldt, n, c, nullptr, (const float *)gf.ptr, nullptr, (const float *)stats.ptr, x.ld));
         gi[0] = x;
         return MCB_OK;
     });
@@ -1851,7 +1886,7 @@ mcb_status Model::loss(const Var &input, const Var &target, Var *out) {
     }
     Var nf = n1, logits;
     if (layers == 0) MCB_TRY(f_layer_norm(x, P[pi + 0], P[pi + 1], eps, &nf));
-    MCB_TRY(f_linear(nf, P[pi + 2], nullptr, &logits));
+    MCB_TRY(f_linear_impl(nf, P[pi + 2], nullptr, MCB_ACT_NONE, &logits, true)); // its only reader is the loss head below
     return f_sce_consuming(logits, tgt, out);
 }
 

@@ -29,6 +29,10 @@ struct Tensor {
     int dt = MCB_F32;
     std::vector<int64_t> shape;
     bool defined = false;
+    // Elements between consecutive rows when they are more than the last extent (a 16-bit matrix whose column count is not a
+    // multiple of 8, kept at the pitch the tensor-core kernels need); 0 = contiguous.  Only the loss head of the decoder and
+    // the backward of the Linear in front of it ever see such a tensor.
+    int64_t ld = 0;
     // Optional by-products of the kernel that wrote an f32 gradient: the same values rounded to bf16 and their
     // column sums.  Valid only while the values are unchanged: whoever modifies the tensor in place drops it.
     std::shared_ptr<GradAux> aux;

@@ -108,7 +108,7 @@ mcb_status mcb_softmax_rows(mcb_ctx *ctx, int mode, const float *a, const float 
 // reduce.cu
 mcb_status mcb_sce_grad(mcb_ctx *ctx, const void *logits, void *out, int32_t dt, const void *labels, int32_t label_dt,
                         int64_t n, int64_t c, float *loss_out, const float *upstream, float *stats_out = nullptr,
-                        const float *stats_in = nullptr); // stats: [n][2] row maximum and sum of exp, passed from the loss pass to the gradient pass
+                        const float *stats_in = nullptr, int64_t ld = 0); // ld: elements between rows (0 = c; a multiple of 8 above c for 16-bit rows).  stats: [n][2] row maximum and sum of exp, passed from the loss pass to the gradient pass
 mcb_status mcb_sum_scaled(mcb_ctx *ctx, const float *x, int64_t n, double scale, float *out);
 // elementwise.cu
 // out[i] = (*scalar) * factor for all i (broadcast of a device scalar)
@@ -122,6 +122,8 @@ mcb_status mcb_add_typed(mcb_ctx *ctx, const void *a, int32_t a_dt, const void *
 // Returns MCB_UNSUPPORTED (nothing launched) unless cols % 8 == 0 and all pointers are 16-byte aligned.
 mcb_status mcb_map_colsum(mcb_ctx *ctx, int mode, const void *a, const void *b, void *out_bf16, int64_t rows, int64_t cols,
                           float *colsum_out, int32_t lp_dt = MCB_BF16); // lp_dt: the 16-bit type of out (and of a, b in modes 1, 2)
+// layout.cu: copies a 16-bit [rows, cols] matrix between row pitches; columns between cols and dst_ld are zero
+mcb_status mcb_repitch16(mcb_ctx *ctx, const void *src, int64_t src_ld, void *dst, int64_t dst_ld, int64_t rows, int64_t cols);
 bool mcb_map_colsum_supported(const void *a, const void *b, const void *out, int64_t cols);
 // reduce.cu: out[col] = sum of `parts` rows of partial[parts, cols], fixed order
 mcb_status mcb_partial_sum_final(mcb_ctx *ctx, const float *partial, int parts, int64_t cols, float *out);

@@ -43,7 +43,39 @@ __global__ void permute_kernel(const float *__restrict__ a, float *__restrict__ 
     }
 }
 
+// one thread per group of eight columns of the wider-pitched side: that side (16-byte aligned rows) in one access
+__global__ void repitch16_kernel(const uint16_t *__restrict__ src, long long src_ld, uint16_t *__restrict__ dst, long long dst_ld, long long rows, int cols) {
+    dep_wait();
+    dep_trigger();
+    const int groups = (cols + 7) / 8;
+    const bool pad = dst_ld > cols;
+    const long long total = rows * groups, stride = (long long)gridDim.x * blockDim.x;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
+        const long long r = i / groups;
+        const int c = (int)(i - r * groups) * 8;
+        __align__(16) uint16_t v[8];
+        if (pad) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = c + q < cols ? src[r * src_ld + c + q] : (uint16_t)0;
+            *reinterpret_cast<uint4 *>(dst + r * dst_ld + c) = *reinterpret_cast<const uint4 *>(v);
+        } else {
+            *reinterpret_cast<uint4 *>(v) = *reinterpret_cast<const uint4 *>(src + r * src_ld + c);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (c + q < cols) dst[r * dst_ld + c + q] = v[q];
+        }
+    }
+}
+
 } // namespace
+
+mcb_status mcb_repitch16(mcb_ctx *ctx, const void *src, int64_t src_ld, void *dst, int64_t dst_ld, int64_t rows, int64_t cols) {
+    if (rows == 0 || cols == 0) return MCB_OK;
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, repitch16_kernel, dim3(mcb_grid_for(ctx, rows * ((cols + 7) / 8), 256, 8)), dim3(256), 0, (const uint16_t *)src,
+                                 (long long)src_ld, (uint16_t *)dst, (long long)dst_ld, (long long)rows, (int)cols));
+    ctx->launches++;
+    return MCB_OK;
+}
 
 extern "C" {
 

@@ -413,17 +413,18 @@ template <> __device__ __forceinline__ uint32_t lp_pack<float>(float, float) { r
 
 // per-thread online (max, sum) merged across the block
 template <typename T>
-__device__ __forceinline__ void row_max_sumexp(const T *__restrict__ row, long long c, float *red, float &mx_out,
+__device__ __forceinline__ void row_max_sumexp(const T *__restrict__ row, long long c, long long ld, float *red, float &mx_out,
                                                float &sum_out) {
     float m = -INFINITY, s = 0.0f;
     // 4 elements per load when the row is wide and aligned: one running-max update per group
     bool vec = ((c & 3) == 0) && ((reinterpret_cast<uintptr_t>(row) & (4 * sizeof(T) - 1)) == 0);
-    bool vec8 = sizeof(T) == 2 && ((c & 7) == 0) && ((reinterpret_cast<uintptr_t>(row) & 15) == 0);
+    bool vec8 = sizeof(T) == 2 && ((ld & 7) == 0) && ((reinterpret_cast<uintptr_t>(row) & 15) == 0);
     if (vec8) {
         // bf16 rows: 16-byte loads, 8 logits per thread per step
         const uint4 *r8 = reinterpret_cast<const uint4 *>(row);
+        const long long whole = c >> 3;
 #pragma unroll 4
-        for (long long j = threadIdx.x; j < (c >> 3); j += blockDim.x) {
+        for (long long j = threadIdx.x; j < ((c + 7) >> 3); j += blockDim.x) {
             uint4 raw = r8[j];
             float f[8];
             unsigned wds[4] = {raw.x, raw.y, raw.z, raw.w};
@@ -432,6 +433,11 @@ __device__ __forceinline__ void row_max_sumexp(const T *__restrict__ row, long l
                 const float2 pr = lp_unpack<T>(wds[q]);
                 f[2 * q] = pr.x;
                 f[2 * q + 1] = pr.y;
+            }
+            if (j >= whole) { // the last group of a row whose length is no multiple of 8 (at least one logit is there)
+#pragma unroll
+                for (int q = 1; q < 8; ++q)
+                    if (j * 8 + q >= c) f[q] = -INFINITY;
             }
             float gm = fmaxf(fmaxf(fmaxf(f[0], f[1]), fmaxf(f[2], f[3])), fmaxf(fmaxf(f[4], f[5]), fmaxf(f[6], f[7])));
             if (gm > m) {
@@ -490,7 +496,7 @@ __global__ void sce_rows_kernel(const float *__restrict__ x, const void *__restr
     }
     const float *row = x + i * c;
     float mx, sum;
-    row_max_sumexp<float>(row, c, red, mx, sum);
+    row_max_sumexp<float>(row, c, c, red, mx, sum);
     if (threadIdx.x == 0) row_loss[i] = (mx + logf(sum)) - row[lab];
 }
 __global__ void sce_final_kernel(const float *__restrict__ row_loss, long long n, float *__restrict__ loss) {
@@ -512,12 +518,12 @@ __global__ void sce_final_kernel(const float *__restrict__ row_loss, long long n
 template <typename T>
 __global__ void __launch_bounds__(512, 3) sce_fused_kernel(const T *x, T *out, const void *__restrict__ labels, int label_dt, long long n,
                                  long long c, float *__restrict__ row_loss, const float *__restrict__ upstream,
-                                 unsigned int *err, float *__restrict__ stats_out, const float *__restrict__ stats_in) {
+                                 unsigned int *err, float *__restrict__ stats_out, const float *__restrict__ stats_in, long long ld) {
     __shared__ float red[32];
     long long i = blockIdx.x;
     long long lab = load_index(labels, label_dt, i);
-    const T *row = x + i * c;
-    T *orow = out + i * c;
+    const T *row = x + i * ld;
+    T *orow = out + i * ld;
     if (lab < 0 || lab >= c) {
         if (threadIdx.x == 0) {
             atomicOr(err, MCB_DEVERR_LABEL);
@@ -532,7 +538,7 @@ __global__ void __launch_bounds__(512, 3) sce_fused_kernel(const T *x, T *out, c
         mx = stats_in[2 * i];
         sum = stats_in[2 * i + 1];
     } else {
-        row_max_sumexp<T>(row, c, red, mx, sum);
+        row_max_sumexp<T>(row, c, ld, red, mx, sum);
     }
     if (row_loss) { // the label's logit is read before anyone overwrites it
         float at_label = Elem<T>::ld(row, lab);
@@ -547,13 +553,13 @@ __global__ void __launch_bounds__(512, 3) sce_fused_kernel(const T *x, T *out, c
     float up = upstream ? upstream[0] : 1.0f;
     float inv_sum = 1.0f / sum, k = up / (float)n;
     bool vec = ((c & 3) == 0) && (((reinterpret_cast<uintptr_t>(row) | reinterpret_cast<uintptr_t>(orow)) & (4 * sizeof(T) - 1)) == 0);
-    const bool vec8 = sizeof(T) == 2 && ((c & 7) == 0) && (((reinterpret_cast<uintptr_t>(row) | reinterpret_cast<uintptr_t>(orow)) & 15) == 0);
+    const bool vec8 = sizeof(T) == 2 && ((ld & 7) == 0) && (((reinterpret_cast<uintptr_t>(row) | reinterpret_cast<uintptr_t>(orow)) & 15) == 0);
     if (vec8) {
         // bf16 rows: 16-byte loads and stores, 8 logits per thread per step, several steps in flight
         const uint4 *r8 = reinterpret_cast<const uint4 *>(row);
         uint4 *o8 = reinterpret_cast<uint4 *>(orow);
 #pragma unroll 4
-        for (long long j = threadIdx.x; j < (c >> 3); j += blockDim.x) {
+        for (long long j = threadIdx.x; j < ((c + 7) >> 3); j += blockDim.x) { // (what follows the row up to its pitch is nobody's)
             const uint4 raw = r8[j];
             const unsigned wds[4] = {raw.x, raw.y, raw.z, raw.w};
             float p[8];
@@ -604,7 +610,7 @@ __global__ void __launch_bounds__(512, 3) sce_fused_kernel(const T *x, T *out, c
 // p = 2^(v * log2e - (mx * log2e + log2(sum))).  `out` may alias `x`: a chunk is written by the thread that read it.
 template <typename T>
 __global__ void __launch_bounds__(256) sce_grad_stream_kernel(const uint4 *x, uint4 *out, const void *__restrict__ labels, int label_dt,
-                                                              long long n, long long c8, const float *__restrict__ stats,
+                                                              long long n, long long c, long long c8, const float *__restrict__ stats,
                                                               const float *__restrict__ upstream, unsigned int *err) {
     const long long row = blockIdx.y;
     const long long j0 = (long long)blockIdx.x * 1024 + threadIdx.x;
@@ -619,7 +625,7 @@ __global__ void __launch_bounds__(256) sce_grad_stream_kernel(const uint4 *x, ui
         raw[u] = j < c8 ? r8[j] : make_uint4(0u, 0u, 0u, 0u);
     }
     const long long lab = load_index(labels, label_dt, row);
-    const bool bad = lab < 0 || lab >= c8 * 8;
+    const bool bad = lab < 0 || lab >= c;
     if (bad && blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, MCB_DEVERR_LABEL);
     const float mx = stats[2 * row], sum = stats[2 * row + 1];
     const float k = (upstream ? upstream[0] : 1.0f) / (float)n;
@@ -1038,7 +1044,8 @@ mcb_status mcb_embedding_backward(mcb_ctx *ctx, const void *ids, int32_t id_dt, 
 
 // gradient of the mean cross entropy (times *upstream), optionally with the loss, in one pass
 mcb_status mcb_sce_grad(mcb_ctx *ctx, const void *logits, void *out, int32_t dt, const void *labels, int32_t label_dt,
-                        int64_t n, int64_t c, float *loss_out, const float *upstream, float *stats_out, const float *stats_in) {
+                        int64_t n, int64_t c, float *loss_out, const float *upstream, float *stats_out, const float *stats_in, int64_t ld) {
+    if (ld == 0) ld = c;
     if (!index_dtype_ok(label_dt)) return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "labels must be i64, i32 or u8");
     if (n == 0) return loss_out ? mcb_memset(ctx, loss_out, 0, sizeof(float)) : MCB_OK;
     if (c == 0) return MCB_OK;
@@ -1047,26 +1054,26 @@ mcb_status mcb_sce_grad(mcb_ctx *ctx, const void *logits, void *out, int32_t dt,
     int threads = c >= 4096 ? 512 : (c >= 256 ? 128 : 32);
     // algorithmic bytes: one read of the logits, one write of the gradient when requested
     ProfScope prof(ctx, MCB_PROF_LOSS, 0.0, (double)n * c * (mcb_is_lp(dt) ? 2.0 : 4.0) * (out ? 2.0 : 1.0) + 8.0 * n);
-    if (mcb_is_lp(dt) && out && stats_in && !loss_out && !stats_out && (c % 8) == 0 && n <= 65535 && mcb_aligned16(logits) && mcb_aligned16(out) &&
+    if (mcb_is_lp(dt) && out && stats_in && !loss_out && !stats_out && (ld % 8) == 0 && ld - c < 8 && n <= 65535 && mcb_aligned16(logits) && mcb_aligned16(out) &&
         !knob_on(ctx, K_SCE_NO_STREAM)) {
         // gradient pass with known row statistics: pure streaming
-        const long long c8 = c / 8;
+        const long long c8 = ld / 8;
         dim3 grid((unsigned)((c8 + 1023) / 1024), (unsigned)n);
         if (dt == MCB_BF16)
             MCB_CUDA(ctx, mcb_launch_dep(ctx, sce_grad_stream_kernel<__nv_bfloat16>, grid, dim3(256), 0, (const uint4 *)logits, (uint4 *)out, labels,
-                                         (int)label_dt, (long long)n, c8, stats_in, upstream, ctx->d_err));
+                                         (int)label_dt, (long long)n, (long long)c, c8, stats_in, upstream, ctx->d_err));
         else
             MCB_CUDA(ctx, mcb_launch_dep(ctx, sce_grad_stream_kernel<__half>, grid, dim3(256), 0, (const uint4 *)logits, (uint4 *)out, labels,
-                                         (int)label_dt, (long long)n, c8, stats_in, upstream, ctx->d_err));
+                                         (int)label_dt, (long long)n, (long long)c, c8, stats_in, upstream, ctx->d_err));
         MCB_LAUNCHED(ctx);
         return MCB_OK;
     }
     if (dt == MCB_F32)
-        sce_fused_kernel<float><<<(unsigned)n, threads, 0, ctx->stream>>>((const float *)logits, (float *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in);
+        sce_fused_kernel<float><<<(unsigned)n, threads, 0, ctx->stream>>>((const float *)logits, (float *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld);
     else if (dt == MCB_BF16)
-        sce_fused_kernel<__nv_bfloat16><<<(unsigned)n, threads, 0, ctx->stream>>>((const __nv_bfloat16 *)logits, (__nv_bfloat16 *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in);
+        sce_fused_kernel<__nv_bfloat16><<<(unsigned)n, threads, 0, ctx->stream>>>((const __nv_bfloat16 *)logits, (__nv_bfloat16 *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld);
     else if (dt == MCB_F16)
-        sce_fused_kernel<__half><<<(unsigned)n, threads, 0, ctx->stream>>>((const __half *)logits, (__half *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in);
+        sce_fused_kernel<__half><<<(unsigned)n, threads, 0, ctx->stream>>>((const __half *)logits, (__half *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld);
     else
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "logits must be f32, bf16 or f16");
     MCB_LAUNCHED(ctx);

@@ -424,6 +424,48 @@ def test_encoder_block_amp_c2_reduced(mc, ctx, oracle, lowp):
     amp_step(mc, ctx, oracle, "encoder", [d, heads, ff, 0], lambda: oracle.EncoderBlock(d, heads, ff), x, t, {5}, lowp=lowp)
 
 
+# a vocabulary that is no multiple of 8 (logits at a padded row pitch: one and seven columns short of it) and heads that are
+# not 64 wide; same limits as the sizes below
+@pytest.mark.parametrize("lowp", ["bf16", "f16"])
+@pytest.mark.parametrize("vocab,d,heads", [(511, 128, 4), (513, 192, 2)])
+def test_decoder_amp_odd_vocab(mc, ctx, oracle, vocab, d, heads, lowp):
+    rng = np.random.default_rng(1240)
+    ff, layers, s, b = 256, 2, 70, 2
+    ids = rng.integers(0, vocab, (b, s)).astype(np.int64)
+    tgt = np.concatenate([ids[:, 1:], rng.integers(0, vocab, (b, 1))], 1).astype(np.int64)
+    amp_step(mc, ctx, oracle, "decoder", [vocab, d, heads, ff, layers, 0], lambda: oracle.Decoder(vocab, d, heads, ff, layers, 0), ids, tgt,
+             {1 + 16 * l + 5 for l in range(layers)}, lowp=lowp)
+
+
+# linear layers whose output width is no multiple of 8, composed from F.*: forward, all three gradients, with and without
+# the fused activation.  16-bit operands: each output and gradient is an f32 sum rounded once (2^-9 of its size for bf16), the
+# gradients take one more rounding of g (2^-9): 2^-7 of the tensor's maximum leaves a factor of two
+@pytest.mark.parametrize("act", [None, "gelu", "relu"])
+@pytest.mark.parametrize("m,k,n", [(1, 8, 1), (130, 64, 10), (257, 72, 131)])
+def test_linear_autocast_odd_width(mc, ctx, m, k, n, act):
+    rng = np.random.default_rng(m + n)
+    r16 = lambda a: mc.bf16_bits_to_f32(mc.f32_to_bf16_bits(a)).reshape(a.shape)
+    x, w, b, g = (r16(rng.standard_normal(sh).astype(np.float32)) for sh in ((m, k), (n, k), (n,), (m, n)))
+    vx, vw, vb, vg = mc.Variable(ctx, x), mc.Variable(ctx, w), mc.Variable(ctx, b), mc.Variable.constant(ctx, g)
+    F = mc.F
+    with mc.autocast(mc.BF16):
+        y = F.linear(vx, vw, vb) if act is None else F.linear_activation(vx, vw, vb, act)
+    F.sum(F.mul(y, vg)).backward()
+    x64, w64 = x.astype(np.float64), w.astype(np.float64)
+    pre = x64 @ w64.T + b
+    p16 = r16(pre.astype(np.float32)).astype(np.float64)
+    if act == "gelu":
+        t = np.tanh(0.7978845608028654 * (p16 + 0.044715 * p16 ** 3))
+        yr = 0.5 * p16 * (1 + t)
+        gr = g * (0.5 * (1 + t) + 0.5 * p16 * (1 - t * t) * 0.7978845608028654 * (1 + 3 * 0.044715 * p16 ** 2))
+    elif act == "relu":
+        yr, gr = np.maximum(p16, 0), g * (p16 > 0)
+    else:
+        yr, gr = pre, g.astype(np.float64)
+    for got, ref in ((y.data, yr), (vx.grad, gr @ w64), (vw.grad, gr.T @ x64), (vb.grad, gr.sum(0))):
+        assert np.abs(got - ref).max() <= 2.0 ** -7 * max(np.abs(ref).max(), 1e-3)
+
+
 @pytest.mark.parametrize("lowp", ["bf16", "f16"])
 def test_decoder_amp_c4_reduced(mc, ctx, oracle, lowp):
     rng = np.random.default_rng(1239)
