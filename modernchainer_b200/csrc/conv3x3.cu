@@ -1,0 +1,391 @@
+// 3 x 3 convolution with stride 1 (forward, data gradient, weight gradient) in exact f32, as direct convolutions on image rows
+// kept in shared memory: each input element is fetched once per CTA for its nine taps, where the implicit GEMM
+// (conv_simt.cu) gathers it nine times.
+//
+// Pixels are taken in groups of four neighbours of an output row; a CTA takes 32 or 64 consecutive groups of the flattened
+// (sample, row, group) order, whatever rows and samples they span.  Their input rows are one contiguous range of VIRTUAL rows:
+// sample n contributes oh + 2 of them, the rows y - pad .. of its image with zero rows where the window leaves it.
+// Shapes that leave the SMs idle otherwise (14 x 14 images, 20 channels, 4 samples) so lose only the rounding of a row to
+// groups of four and of the channels to eight.
+//
+// Bound by the FMA pipe: per source channel and kernel row a thread spends 96 packed FMAs (8 channels x 8 pixels x 3 taps) on
+// 6 + 4 shared-memory loads.
+#include <algorithm>
+
+#include "internal.h"
+#include "simt_tile.cuh"
+
+namespace {
+
+using namespace simt;
+
+struct Rows { // geometry shared by the kernels
+    int oh, ow, s4;        // output rows, columns, groups of four per row
+    int h, w, pad;         // source image
+    int pitch;             // floats per virtual row in shared memory
+    int groups;            // n * oh * s4
+    int vrows;             // virtual rows of a CTA at most
+};
+
+struct Conv3Args {
+    Rows r;
+    const float *wt, *src, *bias;
+    float *out;
+    int M, C;              // output and source channels of this product
+    int bm;                // output channels per CTA: 8 x warps
+    int a_m, a_ch;         // W strides: per output channel, per source channel
+};
+
+constexpr int CC = 4;      // source channels per stage
+
+// virtual row of a group's first tap row
+__device__ __forceinline__ int group_row(const Rows &r, int g, int &n, int &y, int &s) {
+    const int line = g / r.s4;
+    s = g - line * r.s4;
+    n = line / r.oh;
+    y = line - n * r.oh;
+    return n * (r.oh + 2) + y;
+}
+
+// where the virtual rows of a CTA come from, worked out once (divisions): element offset of (sample, channel 0, row y, column -pad),
+// or -1 for a row outside the image
+__device__ __forceinline__ void map_rows(const Rows &r, long long *from, int C, int v0, int rows) {
+    for (int v = threadIdx.x; v < rows; v += blockDim.x) {
+        const int n = (v0 + v) / (r.oh + 2), y = (v0 + v) - n * (r.oh + 2) - r.pad;
+        from[v] = (unsigned)y < (unsigned)r.h ? ((long long)n * C * r.h + y) * r.w : -1;
+    }
+}
+// the mapped rows of channels [c0, c0 + nc) into dst[channel][row][pitch]; a warp takes a row at a time
+__device__ __forceinline__ void load_rows(const Rows &r, float *dst, int plane, const float *src, const long long *from, int c0, int nc, int rows) {
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const long long cplane = (long long)r.h * r.w;
+    for (int v = threadIdx.x >> 5; v < rows; v += warps) {
+        const long long at = from[v];
+        for (int x = lane; x < r.pitch; x += 32) {
+            const bool ok = at >= 0 && (unsigned)(x - r.pad) < (unsigned)r.w;
+            const float *sp = ok ? src + at + c0 * cplane + (x - r.pad) : src;
+            const long long step = ok ? cplane : 0;
+            unsigned d = smem_u32(dst + v * r.pitch + x);
+            for (int c = 0; c < nc; ++c, sp += step, d += plane * 4) cp4(d, sp, ok ? 4 : 0);
+        }
+    }
+}
+
+// Warp w of a CTA owns output channels m0 + 8 w .., lane l the groups g0 + l (and g0 + 32 + l).  FLIP: taps in reverse order (the
+// data gradient as a convolution of g).
+template <bool FLIP, int GP> __global__ void __launch_bounds__(256) conv3x3_kernel(const Conv3Args p) {
+    extern __shared__ __align__(16) float smem[];
+    const Rows r = p.r;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int g0 = blockIdx.x * (32 * GP), m0 = blockIdx.y * p.bm, wp = p.bm + 4;
+    const int plane = r.vrows * r.pitch, stage = CC * plane + CC * 9 * wp;
+    long long *from = reinterpret_cast<long long *>(smem + 2 * stage);
+    int off[GP], gn[GP], gy[GP], gs[GP];
+    int n, y, s;
+    const int v0 = group_row(r, g0, n, y, s);
+    const int rows = group_row(r, min(g0 + 32 * GP, r.groups) - 1, n, y, s) + 3 - v0;
+#pragma unroll
+    for (int j = 0; j < GP; ++j) {
+        const int v = group_row(r, min(g0 + lane + 32 * j, r.groups - 1), gn[j], gy[j], gs[j]);
+        off[j] = (v - v0) * r.pitch + 4 * gs[j];
+    }
+    unsigned long long acc[4][4 * GP]; // channel pairs x pixels
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4 * GP; ++j) acc[i][j] = 0ull;
+    map_rows(r, from, p.C, v0, rows);
+    __syncthreads();
+    dep_wait();
+    dep_trigger();
+    const int chunks = (p.C + CC - 1) / CC;
+    auto fetch = [&](int i) {
+        if (i < chunks) {
+            float *xs = smem + (i & 1) * stage;
+            const int c0 = i * CC, nc = min(CC, p.C - c0);
+            load_rows(r, xs, plane, p.src, from, c0, nc, rows);
+            const unsigned wd = smem_u32(xs + CC * plane);
+            for (int e = threadIdx.x; e < p.bm * CC * 9; e += blockDim.x) { // W as [channel][tap][output channel]
+                const int m = e / (CC * 9), ct = e - m * (CC * 9), c = ct / 9, t = ct - c * 9;
+                const bool ok = m0 + m < p.M && c < nc;
+                cp4(wd + (unsigned)(ct * wp + m) * 4, ok ? p.wt + (long long)(m0 + m) * p.a_m + (long long)(c0 + c) * p.a_ch + (FLIP ? 8 - t : t) : p.wt,
+                    ok ? 4 : 0);
+            }
+        }
+        cp_commit();
+    };
+    fetch(0);
+    for (int i = 0; i < chunks; ++i) {
+        fetch(i + 1);
+        cp_wait<1>();
+        __syncthreads();
+        const float *xs = smem + (i & 1) * stage, *ws = xs + CC * plane + warp * 8;
+        const int nc = min(CC, p.C - i * CC);
+        for (int c = 0; c < nc; ++c) {
+#pragma unroll
+            for (int ky = 0; ky < 3; ++ky) {
+                unsigned long long x2[GP][6];
+#pragma unroll
+                for (int j = 0; j < GP; ++j) {
+                    const float *row = xs + c * plane + off[j] + ky * r.pitch;
+                    const float4 a = *reinterpret_cast<const float4 *>(row);
+                    const float2 b = *reinterpret_cast<const float2 *>(row + 4);
+                    x2[j][0] = pack2(a.x, a.x), x2[j][1] = pack2(a.y, a.y), x2[j][2] = pack2(a.z, a.z), x2[j][3] = pack2(a.w, a.w);
+                    x2[j][4] = pack2(b.x, b.x), x2[j][5] = pack2(b.y, b.y);
+                }
+#pragma unroll
+                for (int kx = 0; kx < 3; ++kx) {
+                    const ulonglong2 *w2 = reinterpret_cast<const ulonglong2 *>(ws + (c * 9 + ky * 3 + kx) * wp);
+                    const ulonglong2 wa = w2[0], wb = w2[1];
+#pragma unroll
+                    for (int j = 0; j < GP; ++j)
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            fma2(acc[0][j * 4 + q], wa.x, x2[j][q + kx]);
+                            fma2(acc[1][j * 4 + q], wa.y, x2[j][q + kx]);
+                            fma2(acc[2][j * 4 + q], wb.x, x2[j][q + kx]);
+                            fma2(acc[3][j * 4 + q], wb.y, x2[j][q + kx]);
+                        }
+                }
+            }
+        }
+        __syncthreads(); // the stage is free for the fetch of the next round
+    }
+    cp_wait<0>();
+#pragma unroll
+    for (int j = 0; j < GP; ++j) {
+        if (g0 + lane + 32 * j >= r.groups) continue;
+        const int x = 4 * gs[j];
+        const bool vec = (r.ow & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int m = m0 + warp * 8 + i;
+            if (m >= p.M) break;
+            const float b = p.bias ? p.bias[m] : 0.0f;
+            float v[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float lo, hi;
+                unpack2(acc[i / 2][j * 4 + q], lo, hi);
+                v[q] = ((i & 1) ? hi : lo) + b;
+            }
+            float *o = p.out + (((long long)gn[j] * p.M + m) * r.oh + gy[j]) * r.ow + x;
+            if (vec) {
+                *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (x + q < r.ow) o[q] = v[q];
+            }
+        }
+    }
+}
+
+// ------------------------------------------------------------------ weight gradient
+// A lane owns one source channel (of CL, a power of two) and one of 32 / CL parts of the groups, its warp four output channels:
+// acc[o][tap] as even- and odd-pixel sums.  Per group of four pixels 72 packed FMAs on 4 (g) + 6 (three rows of x) loads.
+// A CTA walks `tiles` tiles of 64 groups and leaves its partial sums in the workspace, which conv_dw_final_kernel adds in order.
+struct Conv3DwArgs {
+    Rows r;
+    const float *x, *g;
+    float *ws;             // [splits][O * C * 9 + O]
+    int O, C, cl, log_cl;  // cl source channels per CTA
+    int tiles;             // tiles of 64 groups per CTA
+    int xplane;            // floats per channel in shared memory, 4 mod 32: eight lanes' 128-bit loads fall into different banks
+};
+constexpr int DG = 64;         // groups per tile
+constexpr int GP4 = DG * 4 + 4; // floats per output channel of g in shared memory
+
+__global__ void __launch_bounds__(256) conv3x3_dw_kernel(const Conv3DwArgs p) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int offs[DG], left[DG]; // a group's first tap in xs, its columns inside the row
+    __shared__ long long gfrom[DG];    // and its first value in g, output channel 0
+    const Rows r = p.r;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    const int o0 = blockIdx.y * (4 * warps), c0 = blockIdx.z * p.cl;
+    const int ch = lane & (p.cl - 1), part = lane >> p.log_cl, parts = 32 >> p.log_cl;
+    float *xs = smem, *gs = smem + p.cl * p.xplane;
+    long long *from = reinterpret_cast<long long *>(gs + 4 * warps * GP4);
+    const bool want_db = blockIdx.z == 0;
+    unsigned long long acc[4][9];
+    float db[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int t = 0; t < 9; ++t) acc[i][t] = 0ull;
+    dep_wait();
+    dep_trigger();
+    const int nc = min(p.cl, p.C - c0);
+    for (int tile = 0; tile < p.tiles; ++tile) {
+        const int g0 = (blockIdx.x * p.tiles + tile) * DG;
+        if (g0 >= r.groups) break;
+        int n, y, s;
+        const int v0 = group_row(r, g0, n, y, s);
+        const int rows = group_row(r, min(g0 + DG, r.groups) - 1, n, y, s) + 3 - v0;
+        __syncthreads(); // the previous tile has been used
+        map_rows(r, from, p.C, v0, rows);
+        for (int i = threadIdx.x; i < DG; i += blockDim.x) {
+            const int v = group_row(r, min(g0 + i, r.groups - 1), n, y, s);
+            offs[i] = (v - v0) * r.pitch + 4 * s;
+            left[i] = g0 + i < r.groups ? r.ow - 4 * s : 0;
+            gfrom[i] = ((long long)n * p.O * r.oh + y) * r.ow + 4 * s;
+        }
+        __syncthreads();
+        load_rows(r, xs, p.xplane, p.x, from, c0, nc, rows);
+        const long long gplane = (long long)r.oh * r.ow;
+        for (int q = threadIdx.x; q < DG * 4; q += blockDim.x) { // g as [output channel][group][4], zero past a row's end
+            const bool in = (q & 3) < left[q >> 2];
+            const float *gp = in ? p.g + gfrom[q >> 2] + (q & 3) + o0 * gplane : p.g;
+            const long long step = in ? gplane : 0;
+            unsigned d = smem_u32(gs + q);
+            for (int o = 0; o < 4 * warps; ++o, d += GP4 * 4) {
+                const bool ok = in && o0 + o < p.O;
+                cp4(d, ok ? gp + o * step : p.g, ok ? 4 : 0);
+            }
+        }
+        cp_commit();
+        cp_wait<0>();
+        __syncthreads();
+        const float *xc = xs + ch * p.xplane, *gw = gs + warp * 4 * GP4;
+        for (int gi = part; gi < DG; gi += parts) {
+            const float *row = xc + offs[gi];
+            ulonglong2 gv[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) gv[i] = *reinterpret_cast<const ulonglong2 *>(gw + i * GP4 + gi * 4);
+            if (want_db) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float a, b, c, d;
+                    unpack2(gv[i].x, a, b);
+                    unpack2(gv[i].y, c, d);
+                    db[i] += (a + b) + (c + d);
+                }
+            }
+#pragma unroll
+            for (int ky = 0; ky < 3; ++ky) {
+                const float4 a = *reinterpret_cast<const float4 *>(row + ky * r.pitch);
+                const float2 b = *reinterpret_cast<const float2 *>(row + ky * r.pitch + 4);
+                const unsigned long long x01 = pack2(a.x, a.y), x12 = pack2(a.y, a.z), x23 = pack2(a.z, a.w), x34 = pack2(a.w, b.x), x45 = pack2(b.x, b.y);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    fma2(acc[i][ky * 3], gv[i].x, x01);
+                    fma2(acc[i][ky * 3], gv[i].y, x23);
+                    fma2(acc[i][ky * 3 + 1], gv[i].x, x12);
+                    fma2(acc[i][ky * 3 + 1], gv[i].y, x34);
+                    fma2(acc[i][ky * 3 + 2], gv[i].x, x23);
+                    fma2(acc[i][ky * 3 + 2], gv[i].y, x45);
+                }
+            }
+        }
+    }
+    float *ws = p.ws + (long long)blockIdx.x * ((long long)p.O * p.C * 9 + p.O);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int o = o0 + warp * 4 + i;
+#pragma unroll
+        for (int t = 0; t < 9; ++t) {
+            float lo, hi;
+            unpack2(acc[i][t], lo, hi);
+            float v = lo + hi;
+            for (int d = 16; d >= p.cl; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d); // parts of one channel
+            if (part == 0 && ch < nc && o < p.O) ws[((long long)o * p.C + c0 + ch) * 9 + t] = v;
+        }
+        float v = db[i];
+        for (int d = 16; d >= p.cl; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+        if (want_db && lane == 0 && o < p.O) ws[(long long)p.O * p.C * 9 + o] = v;
+    }
+}
+
+Rows make_rows(int64_t n, int64_t h, int64_t w, int64_t pad, int64_t oh, int64_t ow, int groups_per_cta) {
+    Rows r;
+    r.oh = (int)oh; r.ow = (int)ow; r.s4 = (int)((ow + 3) / 4);
+    r.h = (int)h; r.w = (int)w; r.pad = (int)pad;
+    r.pitch = 4 * r.s4 + 4;
+    r.groups = (int)(n * oh * r.s4);
+    // the rows that G consecutive groups can touch: lines of groups, two more per sample they span
+    const int lines = (groups_per_cta + r.s4 - 2) / r.s4 + 1;
+    r.vrows = lines + 2 + 2 * ((lines + r.oh - 2) / r.oh);
+    return r;
+}
+
+template <bool FLIP, int GP> mcb_status launch3(mcb_ctx *ctx, Conv3Args p, size_t limit) {
+    const int warps_all = (p.M + 7) / 8, blocks = (warps_all + 7) / 8, warps = (warps_all + blocks - 1) / blocks;
+    p.bm = warps * 8;
+    const size_t bytes = sizeof(float) * 2 * (size_t)(CC * p.r.vrows * p.r.pitch + CC * 9 * (p.bm + 4)) + sizeof(long long) * p.r.vrows;
+    if (bytes > limit) return MCB_UNSUPPORTED;
+    auto kernel = conv3x3_kernel<FLIP, GP>;
+    MCB_CUDA(ctx, mcb_smem_limit(ctx, kernel, limit));
+    const dim3 grid((unsigned)((p.r.groups + 32 * GP - 1) / (32 * GP)), (unsigned)blocks);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, kernel, grid, dim3(32 * warps), bytes, p));
+    ctx->launches++;
+    return MCB_OK;
+}
+
+constexpr size_t kSmemLimit = 200 * 1024;
+
+template <bool FLIP>
+mcb_status pixels3(mcb_ctx *ctx, const float *wt, const float *src, const float *bias, float *out, int64_t n, int64_t C, int64_t h, int64_t w, int64_t M,
+                   int64_t pad, int64_t oh, int64_t ow, int a_m, int a_ch) {
+    if (pad < 0 || pad > 2 || n * (oh + 2) >= (1ll << 31) || M > 65535 * 64) return MCB_UNSUPPORTED;
+    Conv3Args p;
+    p.wt = wt; p.src = src; p.bias = bias; p.out = out;
+    p.M = (int)M; p.C = (int)C;
+    p.a_m = a_m; p.a_ch = a_ch;
+    // 64 groups per CTA while that gives each SM sixteen warps or more, 32 below (twice the CTAs, half the reuse of W)
+    const long long warps = n * oh * ((ow + 3) / 4) / 64 * ((M + 7) / 8);
+    if (warps >= 16ll * ctx->sm_count) {
+        p.r = make_rows(n, h, w, pad, oh, ow, 64);
+        return launch3<FLIP, 2>(ctx, p, kSmemLimit);
+    }
+    p.r = make_rows(n, h, w, pad, oh, ow, 32);
+    return launch3<FLIP, 1>(ctx, p, kSmemLimit);
+}
+
+} // namespace
+
+// MCB_UNSUPPORTED (nothing launched) where a row does not fit or an extent is out of range; the callers have checked 3 x 3, stride 1
+// and mcb_conv_simt_eligible
+mcb_status mcb_conv3x3_forward(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *out, int64_t n, int64_t c, int64_t h, int64_t wd,
+                               int64_t o, int64_t pad, int64_t oh, int64_t ow) {
+    return pixels3<false>(ctx, w, x, bias, out, n, c, h, wd, o, pad, oh, ow, (int)(c * 9), 9);
+}
+
+mcb_status mcb_conv3x3_dx(mcb_ctx *ctx, const float *g, const float *w, float *dx, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t pad,
+                          int64_t oh, int64_t ow) {
+    return pixels3<true>(ctx, w, g, nullptr, dx, n, o, oh, ow, c, 2 - pad, h, wd, 9, (int)(c * 9));
+}
+
+mcb_status mcb_conv3x3_dw(mcb_ctx *ctx, const float *x, const float *g, float *dw, float *db, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o,
+                          int64_t pad, int64_t oh, int64_t ow) {
+    if (pad < 0 || pad > 2 || n * (oh + 2) >= (1ll << 31)) return MCB_UNSUPPORTED;
+    Conv3DwArgs p;
+    p.r = make_rows(n, h, wd, pad, oh, ow, DG);
+    p.x = x; p.g = g;
+    p.O = (int)o; p.C = (int)c;
+    p.log_cl = 0;
+    while ((1 << p.log_cl) < c && p.log_cl < 5) ++p.log_cl;
+    p.cl = 1 << p.log_cl;
+    p.xplane = (p.r.vrows * p.r.pitch + 27) / 32 * 32 + 4;
+    const int warps_all = (int)((o + 3) / 4), oblocks = (warps_all + 7) / 8, warps = (warps_all + oblocks - 1) / oblocks;
+    const int cblocks = (int)((c + p.cl - 1) / p.cl);
+    const size_t bytes = sizeof(float) * ((size_t)p.cl * p.xplane + (size_t)4 * warps * GP4) + sizeof(long long) * p.r.vrows;
+    if (bytes > kSmemLimit || oblocks > 65535 || cblocks > 65535) return MCB_UNSUPPORTED;
+    const long long tiles = (p.r.groups + DG - 1) / DG;
+    // two to three CTAs are resident per SM (shared memory): one pass over them
+    const long long want = std::max<long long>(1, 3ll * ctx->sm_count / ((long long)oblocks * cblocks));
+    p.tiles = (int)((tiles + want - 1) / want);
+    const long long splits = (tiles + p.tiles - 1) / p.tiles, total = (long long)o * c * 9 + o;
+    void *ws;
+    MCB_TRY(mcb_alloc(ctx, sizeof(float) * (size_t)(splits * total), &ws));
+    p.ws = (float *)ws;
+    cudaError_t e = mcb_smem_limit(ctx, conv3x3_dw_kernel, kSmemLimit);
+    if (e == cudaSuccess)
+        e = mcb_launch_dep(ctx, conv3x3_dw_kernel, dim3((unsigned)splits, (unsigned)oblocks, (unsigned)cblocks), dim3(32 * warps), bytes, p);
+    mcb_status st = mcb_cuda_check(ctx, e, "conv3x3 weight gradient launch");
+    if (st == MCB_OK) {
+        ctx->launches++;
+        st = mcb_conv_dw_final(ctx, (const float *)ws, (int)splits, (long long)o * c * 9, (int)o, dw, db);
+    }
+    mcb_free(ctx, ws); // stream-ordered reuse
+    return st;
+}

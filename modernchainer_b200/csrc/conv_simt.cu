@@ -1,0 +1,373 @@
+// NCHW convolution in exact f32 as implicit GEMMs on the packed-FMA tile (simt_tile.cuh): no column matrix, no layout passes.
+//   forward  out[o, pixel]        = sum_k W[o, k] x[window(pixel), k]          k = (c, ky, kx), pixel = (n, oy, ox)
+//   dgrad    dx[c, pixel]         = sum_k W[o, c, ky, kx] g[o, pixel - tap]     k = (o, ky, kx), pixel = (n, iy, ix)
+//   wgrad    dW[o, (c, ky, kx)]   = sum_pixel g[o, pixel] x[window(pixel), ..]  reduction over n oh ow, split over CTAs
+// The pixel operand is gathered element by element with 4-byte asynchronous copies (out-of-image taps are zero-filled by the
+// copy), neighbouring threads taking neighbouring pixels, so a warp reads runs of an image row; what a tap index k means is
+// worked out once per slab for the whole CTA.  Bound by the FMA pipe (and, for a handful of channels, by the gathers: one copy
+// feeds BM FMAs).
+#include <algorithm>
+
+#include "internal.h"
+#include "simt_tile.cuh"
+
+namespace {
+
+using namespace simt;
+
+struct PixArgs {
+    const float *wt, *src, *bias;
+    float *out;
+    int M, K, N;           // output channels of this product, taps, pixels
+    int khkw, kw;
+    int src_h, src_w, dst_h, dst_w;
+    int stride, pad;
+    int src_c;             // channels of src
+    int a_m, a_ch;         // W strides: per output channel, per source channel
+};
+
+// STAGES slabs in flight; tap[]: {source offset of the channel plane, ky, kx, W offset} of the slab's 16 taps
+template <int BM, int BN, int TM, int TN, bool DX>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) conv_pixels_kernel(const PixArgs p) {
+    using T = Tile<BM, BN, TM, TN, true, false>;
+    constexpr int NT = T::kThreads, STAGES = 3, NCOL = BN / NT;
+    static_assert(BN % NT == 0 && NT >= BK, "whole columns per thread");
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int4 taps[STAGES + 1][BK];
+    const int tid = threadIdx.x, m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int nk = (p.K + BK - 1) / BK;
+    const int src_plane = p.src_h * p.src_w, dst_plane = p.dst_h * p.dst_w;
+    T t;
+    t.init(tid);
+    const float *base[NCOL];
+    int y0[NCOL], x0[NCOL];
+#pragma unroll
+    for (int c = 0; c < NCOL; ++c) {
+        const int pix = min(n0 + tid + c * NT, p.N - 1); // columns past the end repeat the last pixel and are not stored
+        const int n = pix / dst_plane, r = pix - n * dst_plane, y = r / p.dst_w, x = r - y * p.dst_w;
+        base[c] = p.src + (long long)n * p.src_c * src_plane;
+        y0[c] = DX ? y + p.pad : y * p.stride - p.pad;
+        x0[c] = DX ? x + p.pad : x * p.stride - p.pad;
+    }
+    auto make_taps = [&](int s) {
+        if (tid < BK && s < nk) {
+            const int k = s * BK + tid, ch = k / p.khkw, r = k - ch * p.khkw, ky = r / p.kw;
+            int4 e = make_int4(ch * src_plane, ky, r - ky * p.kw, ch * p.a_ch + r);
+            if (k >= p.K) e.y = 1 << 29; // no row of any image: zero-filled
+            taps[s % (STAGES + 1)][tid] = e;
+        }
+    };
+    dep_wait();
+    dep_trigger();
+    auto fetch = [&](int s) {
+        if (s < nk) {
+            float *as = smem + (s % STAGES) * T::kStageFloats, *bs = as + T::kAFloats;
+            const int4 *tp = taps[s % (STAGES + 1)];
+            const unsigned a_at = smem_u32(as), b_at = smem_u32(bs);
+#pragma unroll
+            for (int e = tid; e < BM * BK; e += NT) {
+                const int r = e / BK, k = e % BK;
+                const bool ok = m0 + r < p.M && s * BK + k < p.K;
+                cp4(a_at + (unsigned)(r * KP + k) * 4, ok ? p.wt + (long long)(m0 + r) * p.a_m + tp[k].w : p.wt, ok ? 4 : 0);
+            }
+#pragma unroll 4
+            for (int k = 0; k < BK; ++k) {
+                const int4 e = tp[k];
+#pragma unroll
+                for (int c = 0; c < NCOL; ++c) {
+                    int y, x;
+                    bool ok;
+                    if (DX) {
+                        y = y0[c] - e.y;
+                        x = x0[c] - e.z;
+                        ok = true;
+                        if (p.stride > 1) {
+                            const int ys = y / p.stride, xs = x / p.stride;
+                            ok = y >= 0 && x >= 0 && ys * p.stride == y && xs * p.stride == x;
+                            y = ys;
+                            x = xs;
+                        }
+                        ok = ok && (unsigned)y < (unsigned)p.src_h && (unsigned)x < (unsigned)p.src_w;
+                    } else {
+                        y = y0[c] + e.y;
+                        x = x0[c] + e.z;
+                        ok = (unsigned)y < (unsigned)p.src_h && (unsigned)x < (unsigned)p.src_w;
+                    }
+                    cp4(b_at + (unsigned)(k * (BN + 4) + tid + c * NT) * 4, ok ? base[c] + e.x + y * p.src_w + x : p.src, ok ? 4 : 0);
+                }
+            }
+        }
+        cp_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES; ++s) make_taps(s);
+    __syncthreads();
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) fetch(s);
+    for (int s = 0; s < nk; ++s) {
+        cp_wait<STAGES - 2>();
+        __syncthreads(); // slab s is here; the stage and the taps that are written below are free
+        fetch(s + STAGES - 1);
+        make_taps(s + STAGES);
+        const float *as = smem + (s % STAGES) * T::kStageFloats;
+        t.mma(as, as + T::kAFloats);
+    }
+    cp_wait<0>();
+#pragma unroll
+    for (int j = 0; j < TN; j += 4) { // four neighbouring pixels
+        const int pix = n0 + t.col(j);
+        if (pix >= p.N) continue;
+        const int n = pix / dst_plane, r = pix - n * dst_plane;
+        const bool vec = (dst_plane & 3) == 0 && pix + 3 < p.N && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+#pragma unroll
+        for (int i = 0; i < TM; ++i) {
+            const int m = m0 + t.row(i);
+            if (m >= p.M) continue;
+            const float b = p.bias ? p.bias[m] : 0.0f;
+            float *o = p.out + ((long long)n * p.M + m) * dst_plane + r;
+            if (vec) {
+                *reinterpret_cast<float4 *>(o) = make_float4(t.value(i, j) + b, t.value(i, j + 1) + b, t.value(i, j + 2) + b, t.value(i, j + 3) + b);
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (pix + q >= p.N) break;
+                    const int nn = (pix + q) / dst_plane, rr = pix + q - nn * dst_plane;
+                    p.out[((long long)nn * p.M + m) * dst_plane + rr] = t.value(i, j + q) + b;
+                }
+            }
+        }
+    }
+}
+
+struct DwArgs {
+    const float *x, *g;
+    float *ws;             // [splits][O * N + O]: partial dW and partial bias sums
+    int O, N, K;           // output channels, taps c kh kw, pixels n oh ow
+    int c, h, w, khkw, kw, oh, ow, stride, pad;
+    int per;               // pixels per split, a multiple of 16
+};
+
+template <int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) conv_dw_kernel(const DwArgs p) {
+    using T = Tile<BM, BN, TM, TN, true, true>;
+    constexpr int NT = T::kThreads, STAGES = 3, RA = BM * BK / NT, RB = BN * BK / NT, STEP = NT / BK;
+    static_assert(NT % BK == 0 && BM <= NT, "a thread keeps its pixel of the slab and its rows");
+    extern __shared__ __align__(16) float smem[];
+    const int tid = threadIdx.x, m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int k_begin = blockIdx.z * p.per, k_end = min(p.K, k_begin + p.per), nk = k_end > k_begin ? (k_end - k_begin + BK - 1) / BK : 0;
+    const int plane = p.oh * p.ow, src_plane = p.h * p.w;
+    T t;
+    t.init(tid);
+    const int r0 = tid / BK, kk = tid % BK;
+    int tap_off[RB], tap_y[RB], tap_x[RB]; // this thread's columns (c, ky, kx)
+#pragma unroll
+    for (int i = 0; i < RB; ++i) {
+        const int col = n0 + r0 + i * STEP, ch = col / p.khkw, r = col - ch * p.khkw, ky = r / p.kw;
+        tap_off[i] = ch * src_plane;
+        tap_y[i] = col < p.N ? ky - p.pad : -(1 << 29);
+        tap_x[i] = r - ky * p.kw - p.pad;
+    }
+    // this thread's pixel of the next slab to fetch
+    int q = k_begin + kk, n = q / plane, rem = q - n * plane, oy = rem / p.ow, ox = rem - oy * p.ow;
+    float dbsum = 0.0f;
+    dep_wait();
+    dep_trigger();
+    auto fetch = [&](int s) {
+        if (s < nk) {
+            float *as = smem + (s % STAGES) * T::kStageFloats;
+            const unsigned a_at = smem_u32(as), b_at = smem_u32(as + T::kAFloats);
+            const bool live = q < k_end;
+            const float *gp = p.g + ((long long)n * p.O + m0 + r0) * plane + oy * p.ow + ox;
+#pragma unroll
+            for (int i = 0; i < RA; ++i) {
+                const bool ok = live && m0 + r0 + i * STEP < p.O;
+                cp4(a_at + (unsigned)((r0 + i * STEP) * KP + kk) * 4, ok ? gp + (long long)i * STEP * plane : p.g, ok ? 4 : 0);
+            }
+            const float *xp = p.x + (long long)n * p.c * src_plane;
+            const int iy = oy * p.stride, ix = ox * p.stride;
+#pragma unroll
+            for (int i = 0; i < RB; ++i) {
+                const int y = iy + tap_y[i], x = ix + tap_x[i];
+                const bool ok = live && (unsigned)y < (unsigned)p.h && (unsigned)x < (unsigned)p.w;
+                cp4(b_at + (unsigned)((r0 + i * STEP) * KP + kk) * 4, ok ? xp + tap_off[i] + y * p.w + x : p.x, ok ? 4 : 0);
+            }
+            q += BK;
+            ox += BK;
+            while (ox >= p.ow) {
+                ox -= p.ow;
+                if (++oy == p.oh) {
+                    oy = 0;
+                    ++n;
+                }
+            }
+        }
+        cp_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) fetch(s);
+    for (int s = 0; s < nk; ++s) {
+        cp_wait<STAGES - 2>();
+        __syncthreads();
+        fetch(s + STAGES - 1);
+        const float *as = smem + (s % STAGES) * T::kStageFloats;
+        t.mma(as, as + T::kAFloats);
+        if (blockIdx.x == 0 && tid < BM) { // bias gradient: the slab's sums of g
+            float v = 0.0f;
+#pragma unroll
+            for (int k = 0; k < BK; k += 4) {
+                const float4 f = *reinterpret_cast<const float4 *>(as + tid * KP + k);
+                v += (f.x + f.y) + (f.z + f.w);
+            }
+            dbsum += v;
+        }
+    }
+    cp_wait<0>();
+    float *ws = p.ws + (long long)blockIdx.z * ((long long)p.O * p.N + p.O);
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + t.row(i);
+        if (m >= p.O) continue;
+#pragma unroll
+        for (int j = 0; j < TN; ++j) {
+            const int col = n0 + t.col(j);
+            if (col < p.N) ws[(long long)m * p.N + col] = t.value(i, j);
+        }
+    }
+    if (blockIdx.x == 0 && tid < BM && m0 + tid < p.O) ws[(long long)p.O * p.N + m0 + tid] = dbsum;
+}
+
+// adds the splits in order: eight lanes per element take every eighth split, then meet in a fixed tree
+__global__ void __launch_bounds__(256) conv_dw_final_kernel(const float *__restrict__ ws, int splits, long long n_dw, int o, float *__restrict__ dw, float *__restrict__ db) {
+    dep_wait();
+    dep_trigger();
+    const long long total = n_dw + o;
+    const int lane8 = threadIdx.x & 7;
+    const long long i = (long long)blockIdx.x * 32 + (threadIdx.x >> 3);
+    float v = 0.0f;
+    if (i < total)
+        for (int s = lane8; s < splits; s += 8) v += ws[s * total + i];
+#pragma unroll
+    for (int d = 4; d; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    if (i < total && lane8 == 0) {
+        if (i < n_dw) {
+            if (dw) dw[i] = v;
+        } else if (db) {
+            db[i - n_dw] = v;
+        }
+    }
+}
+
+template <int BM, int BN, int TM, int TN, bool DX> mcb_status launch_pixels(mcb_ctx *ctx, const PixArgs &p) {
+    using T = Tile<BM, BN, TM, TN, true, false>;
+    constexpr size_t bytes = sizeof(float) * 3 * T::kStageFloats;
+    auto kernel = conv_pixels_kernel<BM, BN, TM, TN, DX>;
+    MCB_CUDA(ctx, mcb_smem_limit(ctx, kernel, bytes));
+    const dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)((p.M + BM - 1) / BM));
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, kernel, grid, dim3(T::kThreads), bytes, p));
+    ctx->launches++;
+    return MCB_OK;
+}
+
+// Tile by channels (32 rows while that wastes none or fewer of them) and by what fills the SMs: 128 pixels where that still
+// gives every SM two CTAs.
+template <bool DX> mcb_status run_pixels(mcb_ctx *ctx, const PixArgs &p) {
+    const int m32 = (p.M + 31) / 32 * 32, m64 = (p.M + 63) / 64 * 64;
+    const bool wide = (long long)((p.N + 127) / 128) * ((p.M + 63) / 64) >= 2ll * ctx->sm_count;
+    if (m32 < m64) return wide ? launch_pixels<32, 128, 8, 8, DX>(ctx, p) : launch_pixels<32, 64, 4, 8, DX>(ctx, p);
+    return wide ? launch_pixels<64, 128, 8, 8, DX>(ctx, p) : launch_pixels<64, 64, 8, 8, DX>(ctx, p);
+}
+
+template <int BM, int BN, int TM, int TN> mcb_status launch_dw(mcb_ctx *ctx, DwArgs &p, float *dw, float *db) {
+    using T = Tile<BM, BN, TM, TN, true, true>;
+    constexpr size_t bytes = sizeof(float) * 3 * T::kStageFloats;
+    const long long tiles = (long long)((p.O + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+    // enough slices of the pixels for about six CTAs per SM, none shorter than 128 pixels
+    long long splits = std::max<long long>(1, 6ll * ctx->sm_count / tiles);
+    splits = std::min<long long>(splits, (p.K + 127) / 128);
+    splits = std::min<long long>(splits, 1024);
+    p.per = (int)(((p.K + splits - 1) / splits + BK - 1) / BK * BK);
+    splits = (p.K + p.per - 1) / p.per;
+    const long long total = (long long)p.O * p.N + p.O;
+    void *ws;
+    MCB_TRY(mcb_alloc(ctx, sizeof(float) * (size_t)(splits * total), &ws));
+    p.ws = (float *)ws;
+    auto kernel = conv_dw_kernel<BM, BN, TM, TN>;
+    cudaError_t e = mcb_smem_limit(ctx, kernel, bytes);
+    const dim3 grid((unsigned)((p.N + BN - 1) / BN), (unsigned)((p.O + BM - 1) / BM), (unsigned)splits);
+    if (e == cudaSuccess) e = mcb_launch_dep(ctx, kernel, grid, dim3(T::kThreads), bytes, p);
+    mcb_status st = mcb_cuda_check(ctx, e, "convolution weight gradient launch");
+    if (st == MCB_OK) {
+        ctx->launches++;
+        st = mcb_conv_dw_final(ctx, (const float *)ws, (int)splits, (long long)p.O * p.N, p.O, dw, db);
+    }
+    mcb_free(ctx, ws); // stream-ordered reuse
+    return st;
+}
+
+bool fits(int64_t v) { return v > 0 && v < (1ll << 31) - (1 << 20); }
+
+} // namespace
+
+// dw (n_dw values) and db (o values) from `splits` rows of partial sums, in order; either may be NULL
+mcb_status mcb_conv_dw_final(mcb_ctx *ctx, const float *ws, int splits, long long n_dw, int o, float *dw, float *db) {
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, conv_dw_final_kernel, dim3((unsigned)((n_dw + o + 31) / 32)), dim3(256), 0, ws, splits, n_dw, o, dw, db));
+    ctx->launches++;
+    return MCB_OK;
+}
+
+// 32-bit pixel and tap indices, grid limits
+bool mcb_conv_simt_eligible(int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t oh, int64_t ow) {
+    return fits(n * oh * ow) && fits(n * h * wd) && fits(c * kh * kw) && fits(o * kh * kw) && fits(c * h * wd) && fits(o * oh * ow) && kh < (1 << 20) &&
+           kw < (1 << 20) && o <= 65535 * 32 && c <= 65535 * 32 && h < (1 << 28) && wd < (1 << 28);
+}
+
+mcb_status mcb_conv_simt_forward(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *out, int64_t n, int64_t c, int64_t h,
+                                 int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t stride, int64_t pad, int64_t oh, int64_t ow) {
+    if (kh == 3 && kw == 3 && stride == 1) {
+        mcb_status st = mcb_conv3x3_forward(ctx, x, w, bias, out, n, c, h, wd, o, pad, oh, ow);
+        if (st != MCB_UNSUPPORTED) return st;
+    }
+    PixArgs p;
+    p.wt = w; p.src = x; p.bias = bias; p.out = out;
+    p.M = (int)o; p.K = (int)(c * kh * kw); p.N = (int)(n * oh * ow);
+    p.khkw = (int)(kh * kw); p.kw = (int)kw;
+    p.src_h = (int)h; p.src_w = (int)wd; p.dst_h = (int)oh; p.dst_w = (int)ow;
+    p.stride = (int)stride; p.pad = (int)pad;
+    p.src_c = (int)c;
+    p.a_m = p.K; p.a_ch = p.khkw;
+    return run_pixels<false>(ctx, p);
+}
+
+mcb_status mcb_conv_simt_dx(mcb_ctx *ctx, const float *g, const float *w, float *dx, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t kh,
+                            int64_t kw, int64_t stride, int64_t pad, int64_t oh, int64_t ow) {
+    if (kh == 3 && kw == 3 && stride == 1) {
+        mcb_status st = mcb_conv3x3_dx(ctx, g, w, dx, n, c, h, wd, o, pad, oh, ow);
+        if (st != MCB_UNSUPPORTED) return st;
+    }
+    PixArgs p;
+    p.wt = w; p.src = g; p.bias = nullptr; p.out = dx;
+    p.M = (int)c; p.K = (int)(o * kh * kw); p.N = (int)(n * h * wd);
+    p.khkw = (int)(kh * kw); p.kw = (int)kw;
+    p.src_h = (int)oh; p.src_w = (int)ow; p.dst_h = (int)h; p.dst_w = (int)wd;
+    p.stride = (int)stride; p.pad = (int)pad;
+    p.src_c = (int)o;
+    p.a_m = p.khkw; p.a_ch = (int)(c * kh * kw);
+    return run_pixels<true>(ctx, p);
+}
+
+// dw and db (either may be NULL)
+mcb_status mcb_conv_simt_dw(mcb_ctx *ctx, const float *x, const float *g, float *dw, float *db, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o,
+                            int64_t kh, int64_t kw, int64_t stride, int64_t pad, int64_t oh, int64_t ow) {
+    if (kh == 3 && kw == 3 && stride == 1) {
+        mcb_status st = mcb_conv3x3_dw(ctx, x, g, dw, db, n, c, h, wd, o, pad, oh, ow);
+        if (st != MCB_UNSUPPORTED) return st;
+    }
+    DwArgs p;
+    p.x = x; p.g = g;
+    p.O = (int)o; p.N = (int)(c * kh * kw); p.K = (int)(n * oh * ow);
+    p.c = (int)c; p.h = (int)h; p.w = (int)wd; p.khkw = (int)(kh * kw); p.kw = (int)kw; p.oh = (int)oh; p.ow = (int)ow;
+    p.stride = (int)stride; p.pad = (int)pad;
+    const bool narrow = p.N <= 32;
+    if (p.O <= 32) return narrow ? launch_dw<32, 32, 4, 4>(ctx, p, dw, db) : launch_dw<32, 64, 4, 4>(ctx, p, dw, db);
+    return narrow ? launch_dw<64, 32, 8, 4>(ctx, p, dw, db) : launch_dw<64, 64, 8, 4>(ctx, p, dw, db);
+}

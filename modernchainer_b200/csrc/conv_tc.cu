@@ -300,15 +300,21 @@ void fill_dims(ConvDims &d, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t
 
 } // namespace
 
-// Worth the column matrix and three GEMM launches from about 2^24 multiply-adds on; the output channel count must
-// give 16-byte rows ([M, O] f16: O % 8 == 0) and the extents must fit the kernels' 32-bit indices.
-bool mcb_conv_tc_eligible(mcb_ctx *ctx, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t stride, int64_t pad) {
-    if (knob_on(ctx, K_CONV_DIRECT)) return false; // test knob: keep the direct kernels
+// The output channel count must give 16-byte rows ([M, O] f16: O % 8 == 0) and the extents must fit the kernels' 32-bit indices.
+// Worth it against the FMA-pipe kernels (conv3x3.cu, conv_simt.cu) by the measured cost per output pixel in nanoseconds: those
+// spend 6e-5 per tap and output channel (about 35 TFLOP/s), the column matrix and its GEMM 3.8e-3 per tap, 4.5e-3 per output
+// channel and 0.5 for the passes that depend on neither (64 x 64 channels, 3 x 3, 56 x 56 x 64: 384 us there, 494 here; 64 ->
+// 128 channels, 32 x 32 x 128: 458 and 362; 128 -> 256: 751 and 300).  A data gradient with a stride is always worth it: the
+// FMA kernels visit every tap of every input pixel, most of which no output pixel uses.
+bool mcb_conv_tc_eligible(mcb_ctx *ctx, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t stride, int64_t pad,
+                          bool strided_dx) {
+    if (knob_on(ctx, K_CONV_DIRECT)) return false; // test knob: the element-wise kernels
     if (stride <= 0 || pad < 0 || h + 2 * pad < kh || wd + 2 * pad < kw || o % 8) return false;
     ConvDims d;
     fill_dims(d, n, c, h, wd, o, kh, kw, stride, pad);
     const double macs = (double)d.m * d.k * d.o;
-    return macs >= (double)(1 << 24) && d.m % 8 == 0 && d.m * d.k8 < (1ll << 40) && (long long)n * c * h * wd < (1ll << 40);
+    const bool wins = (strided_dx && stride > 1) || 6.0e-5 * d.k * d.o > 3.8e-3 * d.k + 4.5e-3 * d.o + 0.5;
+    return wins && macs >= (double)(1 << 24) && d.m % 8 == 0 && d.m * d.k8 < (1ll << 40) && (long long)n * c * h * wd < (1ll << 40);
 }
 
 mcb_status mcb_conv_tc_forward(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *out, int64_t n, int64_t c, int64_t h,

@@ -98,11 +98,28 @@ mcb_status mcb_layer_norm_backward_ex(mcb_ctx *ctx, const float *x, const float 
                                       float *dbeta, int64_t rows, int64_t dim);
 // conv_tc.cu: convolution as column matrix + tensor-core GEMMs at f32 accuracy (f16 hi/lo pieces); _eligible says whether a
 // problem is large and regular enough for it
-bool mcb_conv_tc_eligible(mcb_ctx *ctx, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t stride, int64_t pad);
+bool mcb_conv_tc_eligible(mcb_ctx *ctx, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t stride, int64_t pad,
+                          bool strided_dx = false);
 mcb_status mcb_conv_tc_forward(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *out, int64_t n, int64_t c, int64_t h,
                                int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t stride, int64_t pad);
 mcb_status mcb_conv_tc_backward(mcb_ctx *ctx, const float *x, const float *w, const float *g, float *dx, float *dw, int64_t n, int64_t c, int64_t h,
                                 int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t stride, int64_t pad);
+// conv_simt.cu: convolution as implicit GEMM on the f32 FMA pipe; _eligible: the extents fit its 32-bit indices
+bool mcb_conv_simt_eligible(int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t oh, int64_t ow);
+mcb_status mcb_conv_simt_forward(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *out, int64_t n, int64_t c, int64_t h,
+                                 int64_t wd, int64_t o, int64_t kh, int64_t kw, int64_t stride, int64_t pad, int64_t oh, int64_t ow);
+mcb_status mcb_conv_simt_dx(mcb_ctx *ctx, const float *g, const float *w, float *dx, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t kh,
+                            int64_t kw, int64_t stride, int64_t pad, int64_t oh, int64_t ow);
+mcb_status mcb_conv_simt_dw(mcb_ctx *ctx, const float *x, const float *g, float *dw, float *db, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o,
+                            int64_t kh, int64_t kw, int64_t stride, int64_t pad, int64_t oh, int64_t ow); // dw and db: either may be NULL
+mcb_status mcb_conv_dw_final(mcb_ctx *ctx, const float *ws, int splits, long long n_dw, int o, float *dw, float *db);
+// conv3x3.cu: the same products for 3 x 3 kernels with stride 1 as direct convolutions; MCB_UNSUPPORTED (nothing launched) outside their range
+mcb_status mcb_conv3x3_forward(mcb_ctx *ctx, const float *x, const float *w, const float *bias, float *out, int64_t n, int64_t c, int64_t h, int64_t wd,
+                               int64_t o, int64_t pad, int64_t oh, int64_t ow);
+mcb_status mcb_conv3x3_dx(mcb_ctx *ctx, const float *g, const float *w, float *dx, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o, int64_t pad,
+                          int64_t oh, int64_t ow);
+mcb_status mcb_conv3x3_dw(mcb_ctx *ctx, const float *x, const float *g, float *dw, float *db, int64_t n, int64_t c, int64_t h, int64_t wd, int64_t o,
+                          int64_t pad, int64_t oh, int64_t ow);
 // reduce.cu: row softmax (mode 0), its backward from x (1) or from the forward's output y (2)
 mcb_status mcb_softmax_rows(mcb_ctx *ctx, int mode, const float *a, const float *b, float *out, int64_t rows, int64_t cols);
 // reduce.cu

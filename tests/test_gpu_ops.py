@@ -490,6 +490,38 @@ def test_conv2d_tensor_core_path(ops, oracle, shape, wshape, stride, pad):
         ops.ctx.set_knob("MCB_CONV_DIRECT", None)
 
 
+# the direct 3 x 3 kernels (rows that are no multiple of four, one-row images, paddings 0 to 2, groups of pixels that span many
+# samples, channel counts off the tiles of 4, 8 and 32), the implicit GEMM (1 x 1, 5 x 5, strides) and the tensor-core products
+# that the cost rule still picks (80 and more output channels; any strided data gradient).  f32 sums against f64: 4 sqrt(terms)
+# 2^-24 of the largest; the tensor-core path at its 1e-5
+@pytest.mark.parametrize("shape,wshape,stride,pad,tol", [
+    ((3, 1, 1, 1), (1, 1, 3, 3), 1, 1, None), ((2, 3, 5, 7), (9, 3, 3, 3), 1, 1, None), ((70, 5, 4, 4), (33, 5, 3, 3), 1, 1, None), ((2, 33, 9, 30), (70, 33, 3, 3), 1, 0, None),
+    ((2, 4, 6, 65), (8, 4, 3, 3), 1, 2, None), ((5, 6, 11, 10), (17, 6, 1, 1), 1, 0, None), ((2, 3, 12, 13), (10, 3, 5, 5), 2, 2, None), ((40, 40, 14, 14), (40, 40, 3, 3), 1, 1, None),
+    ((8, 32, 24, 24), (96, 32, 3, 3), 1, 1, 1e-5), ((8, 64, 16, 16), (24, 64, 3, 3), 2, 1, 1e-5)])
+def test_conv2d_paths(ops, shape, wshape, stride, pad, tol):
+    import torch
+    x, w, b = randn(*shape), randn(*wshape) * 0.3, randn(wshape[0])
+    xt, wt, bt = (torch.tensor(a, dtype=torch.float64, requires_grad=True) for a in (x, w, b))
+    yt = torch.nn.functional.conv2d(xt, wt, bt, stride, pad)
+    g = randn(*yt.shape)
+    yt.backward(torch.tensor(g, dtype=torch.float64))
+    got = (ops.conv2d(x, w, b, stride, pad),) + tuple(ops.conv2d_backward(x, w, g, stride, pad))
+    taps, pixels = w[0].size, g[:, 0].size
+    for a, r, terms in zip(got, (yt.detach(), xt.grad, wt.grad, bt.grad), (taps, w[:, 0].size, pixels, pixels)):
+        r = r.numpy()
+        assert np.abs(a - r).max() <= (tol or 4.0 * np.sqrt(terms) * 2.0 ** -24) * max(np.abs(r).max(), 1.0)
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 2, 2), (2, 3, 6, 10), (3, 5, 28, 14)])
+def test_max_pool_2x2(ops, oracle, shape):
+    x = np.round(randn(*shape) * 2)  # many ties
+    x[0, 0, 0, 0] = np.inf
+    y = oracle.max_pool2d(x, 2, 2, 0)
+    assert np.array_equal(ops.max_pool2d(x, 2, 2, 0), y)
+    g = randn(*y.shape)
+    assert np.array_equal(ops.max_pool2d_backward(x, g, 2, 2, 0), oracle.max_pool2d_backward(x, g, 2, 2, 0))
+
+
 def test_max_pool_tie_rule(ops, oracle):
     x = randn(3, 4, 8, 8)
     x[0, 0, 0:2, 0:2] = 1.5   # four equal maxima: first of each window row gets the gradient
