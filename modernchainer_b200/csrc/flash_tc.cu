@@ -77,7 +77,7 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     unsigned *tmem_slot = (unsigned *)(bars + 13);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // causal: late query tiles walk the most key tiles, so they are scheduled first
     // (CTAs are dispatched in the order of their linear index, read here as (weight rank, sample*head): all the longest
     // jobs of the grid start first and the shortest fill the tail)
@@ -118,7 +118,7 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_slot;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // only shared and tensor memory so far: this much may overlap the previous kernel of the stream
     dep_wait();
     dep_trigger();
@@ -159,23 +159,24 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const unsigned lead = elect_lane();
             constexpr unsigned idesc_s = make_idesc(BM, BN, 0, 0, F16);   // S = Q K^T: both operands K-major
             constexpr unsigned idesc_o = make_idesc(BM, 64 * NB, 0, 1, F16); // O += P V: V is [keys, columns] = MN-major B, whole blocks of 64
             const unsigned tmem_s = tmem_base + kColS, tmem_o = tmem_base + kColO;
             const unsigned a_q = smem_u32(sQ);
-            bool ok = mbar_wait(q_full, 0, abort_flag, args.err);
+            bool ok = mbar_wait_warp(q_full, 0, abort_flag, args.err);
             auto issue_s = [&](int j) {
                 const unsigned b_k = smem_u32(smem + kSmemKV + (j & 1) * 2 * kTileBytes);
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks) {
                     const unsigned off = (ks >> 2) * kBlockBytes + (ks & 3) * 32;
-                    tc_mma(tmem_s, make_desc(a_q + off, 16, 1024), make_desc(b_k + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u);
+                    tc_mma(tmem_s, make_desc(a_q + off, 16, 1024), make_desc(b_k + off, 16, 1024), idesc_s, ks > 0 ? 1u : 0u, lead);
                 }
-                tc_commit(s_full);
-                tc_commit(&k_empty[j & 1]);
+                tc_commit(s_full, lead);
+                tc_commit(&k_empty[j & 1], lead);
             };
-            if (ok) ok = mbar_wait(&k_full[0], 0, abort_flag, args.err);
+            if (ok) ok = mbar_wait_warp(&k_full[0], 0, abort_flag, args.err);
             if (ok) {
                 tc_fence_after();
                 issue_s(0);
@@ -184,14 +185,14 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 const int st = j & 1;
                 if (j + 1 < nt) {
                     // next scores as soon as their K tile is here and the rows have read the current S
-                    ok = mbar_wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1u, abort_flag, args.err);
-                    if (ok) ok = mbar_wait(s_free, (unsigned)j & 1u, abort_flag, args.err);
+                    ok = mbar_wait_warp(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1u, abort_flag, args.err);
+                    if (ok) ok = mbar_wait_warp(s_free, (unsigned)j & 1u, abort_flag, args.err);
                     if (!ok) break;
                     tc_fence_after();
                     issue_s(j + 1);
                 }
-                ok = mbar_wait(&v_full[st], (unsigned)(j >> 1) & 1u, abort_flag, args.err);
-                if (ok) ok = mbar_wait(p_full, (unsigned)j & 1u, abort_flag, args.err);
+                ok = mbar_wait_warp(&v_full[st], (unsigned)(j >> 1) & 1u, abort_flag, args.err);
+                if (ok) ok = mbar_wait_warp(p_full, (unsigned)j & 1u, abort_flag, args.err);
                 if (!ok) break;
                 tc_fence_after();
                 const unsigned b_v = smem_u32(smem + kSmemKV + st * 2 * kTileBytes + kTileBytes);
@@ -199,10 +200,10 @@ flash_tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 for (int ks = 0; ks < BN / 16; ++ks) {
                     // P from TMEM: 16 keys = 8 columns of packed pairs per step; V: 16 keys = 2048 bytes per step
                     unsigned long long bd = make_desc(b_v + ks * 2048, NB == 1 ? 8192 : kBlockBytes, 1024);
-                    tc_mma_ta(tmem_o, tmem_base + kColP + ks * 8, bd, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+                    tc_mma_ta(tmem_o, tmem_base + kColP + ks * 8, bd, idesc_o, (j > 0 || ks > 0) ? 1u : 0u, lead);
                 }
-                tc_commit(pv_done);
-                tc_commit(&v_empty[st]);
+                tc_commit(pv_done, lead);
+                tc_commit(&v_empty[st], lead);
             }
         }
     } else {

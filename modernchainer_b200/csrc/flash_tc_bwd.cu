@@ -147,7 +147,7 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     unsigned *tmem_slot = (unsigned *)(bars + 11);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int tiles = args.tiles;
 
     if (threadIdx.x == 0) {
@@ -178,7 +178,7 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_slot;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // Only shared and tensor memory so far: this much may overlap the previous kernel of the stream.  The dK/dV
     // kernel (MODE 0) waits here for everything before it.  The recomputing dQ kernel (MODE 1) is launched right behind
     // it, reads the same inputs and writes other bytes, so it needs nothing from MODE 0: it starts on the SMs that MODE 0's
@@ -229,7 +229,8 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
+        {
+            const unsigned lead = elect_lane();
             constexpr unsigned idesc_sd = make_idesc(BT, BT, 0, 0, F16);                       // S, dP: both operands K-major
             constexpr unsigned idesc_acc = make_idesc(BT, 64 * NB, MODE == 0 ? 1 : 0, 1, F16); // MODE 0: A = P^T / dS^T (MN-major); MODE 1: A = dS (K-major)
             const unsigned x0 = smem_u32(sX0), x1 = smem_u32(sX1), p_addr = smem_u32(sP), ds_addr = smem_u32(sDS);
@@ -240,26 +241,26 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks) {
                     const unsigned off = (ks >> 2) * kBlockBytes + (ks & 3) * 32;
-                    tc_mma(tmem_base + kColS, make_desc(a_s + off, 16, 1024), make_desc(b_s + off, 16, 1024), idesc_sd, ks > 0 ? 1u : 0u);
+                    tc_mma(tmem_base + kColS, make_desc(a_s + off, 16, 1024), make_desc(b_s + off, 16, 1024), idesc_sd, ks > 0 ? 1u : 0u, lead);
                 }
 #pragma unroll
                 for (int ks = 0; ks < HD / 16; ++ks) {
                     const unsigned off = (ks >> 2) * kBlockBytes + (ks & 3) * 32;
-                    tc_mma(tmem_base + kColDP, make_desc(a_p + off, 16, 1024), make_desc(b_p + off, 16, 1024), idesc_sd, ks > 0 ? 1u : 0u);
+                    tc_mma(tmem_base + kColDP, make_desc(a_p + off, 16, 1024), make_desc(b_p + off, 16, 1024), idesc_sd, ks > 0 ? 1u : 0u, lead);
                 }
-                tc_commit(sd_full);
+                tc_commit(sd_full, lead);
             };
             Job jb, nx;
             bool have = job_at<MODE>(args, 0, jb);
             bool ok = true;
             unsigned g = 0; // global step counter
             if (have) {
-                ok = mbar_wait(x_full, 0, abort_flag, args.err);
-                if (ok) ok = mbar_wait(&y_full[0], 0, abort_flag, args.err);
+                ok = mbar_wait_warp(x_full, 0, abort_flag, args.err);
+                if (ok) ok = mbar_wait_warp(&y_full[0], 0, abort_flag, args.err);
                 if (ok) {
                     tc_fence_after();
                     issue_sd(0);
-                    if (jb.nt == 1) tc_commit(x_empty); // the job's last S / dP has been issued: the resident pair is free once it has run
+                    if (jb.nt == 1) tc_commit(x_empty, lead); // the job's last S / dP has been issued: the resident pair is free once it has run
                 }
             }
             for (int it = 0; ok && have; ++it) {
@@ -271,24 +272,24 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     const unsigned st = g % ST;
                     auto next_sd = [&]() {
                         // next scores of this job as soon as their streamed pair is here and the rows have read the current ones
-                        ok = mbar_wait(&y_full[(g + 1) % ST], ((g + 1) / ST) & 1u, abort_flag, args.err);
-                        if (ok) ok = mbar_wait(sd_free, g & 1u, abort_flag, args.err);
+                        ok = mbar_wait_warp(&y_full[(g + 1) % ST], ((g + 1) / ST) & 1u, abort_flag, args.err);
+                        if (ok) ok = mbar_wait_warp(sd_free, g & 1u, abort_flag, args.err);
                         if (!ok) return;
                         tc_fence_after();
                         issue_sd(g + 1);
-                        if (t + 2 == jb.nt) tc_commit(x_empty);
+                        if (t + 2 == jb.nt) tc_commit(x_empty, lead);
                     };
                     if (ST == 2 && t + 1 < jb.nt) {
                         next_sd();
                         if (!ok) break;
                     }
-                    ok = mbar_wait(pds_full, g & 1u, abort_flag, args.err);
+                    ok = mbar_wait_warp(pds_full, g & 1u, abort_flag, args.err);
                     if (!ok) break;
                     tc_fence_after();
                     const unsigned y0 = smem_u32(smem + kSmemY + st * 2 * kTileBytes), y1 = y0 + kTileBytes;
                     const unsigned acc = (t > 0) ? 1u : 0u;
                     const bool spill = MODE == 0 && args.ds_out != nullptr;
-                    if (spill) { // dS of this pair to the scratch of the dQ kernel, while the MMAs below read the same tile
+                    if (spill && lead) { // dS of this pair to the scratch of the dQ kernel, while the MMAs below read the same tile
                         const size_t slot = ((size_t)jb.nh * tiles + (size_t)(jb.t_first + t)) * tiles + (size_t)jb.own;
                         bulk_store(args.ds_out + slot * kDsBytes, sDS, kDsBytes);
                         bulk_commit();
@@ -300,13 +301,13 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         for (int ks = 0; ks < BT / 16; ++ks) {
                             const unsigned a_off = (ks >> 2) * 8192 + (ks & 3) * 2048;
                             tc_mma(tmem_base + acc_a, make_desc(p_addr + a_off, 16384, 1024), make_desc(y1 + ks * 2048, NB == 1 ? 8192 : kBlockBytes, 1024), idesc_acc,
-                                   (ks > 0) ? 1u : acc);
+                                   (ks > 0) ? 1u : acc, lead);
                         }
 #pragma unroll
                         for (int ks = 0; ks < BT / 16; ++ks) {
                             const unsigned a_off = (ks >> 2) * 8192 + (ks & 3) * 2048;
                             tc_mma(tmem_base + acc_b, make_desc(ds_addr + a_off, 16384, 1024), make_desc(y0 + ks * 2048, NB == 1 ? 8192 : kBlockBytes, 1024), idesc_acc,
-                                   (ks > 0) ? 1u : acc);
+                                   (ks > 0) ? 1u : acc, lead);
                         }
                     } else {
                         // dQ += dS K: A = dS straight from TMEM (16 keys = 8 columns of packed pairs per step);
@@ -314,11 +315,11 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                         for (int ks = 0; ks < BT / 16; ++ks)
                             tc_mma_ta(tmem_base + acc_a, tmem_base + kColDSt + ks * 8, make_desc(y0 + ks * 2048, 8192, 1024), idesc_acc,
-                                      (ks > 0) ? 1u : acc);
+                                      (ks > 0) ? 1u : acc, lead);
                     }
-                    if (spill) bulk_wait_read0(); // mma_done also tells the rows that dS may be overwritten
-                    tc_commit(mma_done);
-                    tc_commit(&y_empty[st]);
+                    if (spill && lead) bulk_wait_read0(); // mma_done also tells the rows that dS may be overwritten
+                    tc_commit(mma_done, lead);
+                    tc_commit(&y_empty[st], lead);
                     if (ST == 1 && t + 1 < jb.nt) { // the one streamed stage is refilled behind the MMAs just issued
                         next_sd();
                         if (!ok) break;
@@ -326,19 +327,19 @@ flash_tc_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     if (t + 1 == jb.nt && have_next) {
                         // first scores of the NEXT job, queued behind this job's last accumulating MMAs: they run while the
                         // rows write this job's results out
-                        ok = mbar_wait(x_full, (unsigned)(it + 1) & 1u, abort_flag, args.err);
-                        if (ok) ok = mbar_wait(&y_full[(g + 1) % ST], ((g + 1) / ST) & 1u, abort_flag, args.err);
-                        if (ok) ok = mbar_wait(sd_free, g & 1u, abort_flag, args.err);
+                        ok = mbar_wait_warp(x_full, (unsigned)(it + 1) & 1u, abort_flag, args.err);
+                        if (ok) ok = mbar_wait_warp(&y_full[(g + 1) % ST], ((g + 1) / ST) & 1u, abort_flag, args.err);
+                        if (ok) ok = mbar_wait_warp(sd_free, g & 1u, abort_flag, args.err);
                         if (!ok) break;
                         tc_fence_after();
                         issue_sd(g + 1);
-                        if (nx.nt == 1) tc_commit(x_empty);
+                        if (nx.nt == 1) tc_commit(x_empty, lead);
                     }
                 }
                 jb = nx;
                 have = have_next;
             }
-            if (MODE == 0 && args.ds_out) bulk_wait_all();
+            if (MODE == 0 && args.ds_out && lead) bulk_wait_all();
         }
     } else {
         // ------------------------------------------------------------ pair arithmetic and epilogue (warps 2..9)
@@ -525,7 +526,7 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     unsigned long long *full = bars, *empty = bars + kDqStages, *acc_done = bars + 2 * kDqStages;
     unsigned *tmem_slot = (unsigned *)(acc_done + 1);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     const int lin = (int)(blockIdx.y * gridDim.x + blockIdx.x), rank = lin / (int)gridDim.y, nh = lin - rank * (int)gridDim.y;
     const int n = nh / args.heads, h = nh % args.heads;
     const int tiles = (args.seq + BT - 1) / BT;
@@ -554,7 +555,7 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const unsigned tmem_base = *tmem_slot;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     dep_wait(); // the dS tiles come from the kernel before this one
     dep_trigger();
 
@@ -583,22 +584,24 @@ flash_tc_dq_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        // ---- MMA issuer
+        {
+            const unsigned lead = elect_lane();
             constexpr unsigned idesc = make_idesc(BT, 64 * NB, 0, 1, F16); // A = dS (K-major), B = K as loaded ([keys, hd]: MN-major)
             bool ok = true;
             for (int t = 0; t < nt && ok; ++t) {
                 const int st = t % kDqStages;
-                ok = mbar_wait(&full[st], (unsigned)(t / kDqStages) & 1u, abort_flag, args.err);
+                ok = mbar_wait_warp(&full[st], (unsigned)(t / kDqStages) & 1u, abort_flag, args.err);
                 if (!ok) break;
                 tc_fence_after();
                 const unsigned ds_addr = smem_u32(smem + st * kDqStageBytes), k_addr = ds_addr + kDsBytes;
 #pragma unroll
                 for (int ks = 0; ks < BT / 16; ++ks) // 16 keys per step: 32 bytes inside a 64-key block of 16 KB
                     tc_mma(tmem_base, make_desc(ds_addr + (ks >> 2) * 16384 + (ks & 3) * 32, 16, 1024), make_desc(k_addr + ks * 2048, NB == 1 ? 8192 : kBlockBytes, 1024), idesc,
-                           (t > 0 || ks > 0) ? 1u : 0u);
-                tc_commit(&empty[st]);
+                           (t > 0 || ks > 0) ? 1u : 0u, lead);
+                tc_commit(&empty[st], lead);
             }
-            if (ok) tc_commit(acc_done);
+            if (ok) tc_commit(acc_done, lead);
         }
     } else {
         const int wq = warp & 3;

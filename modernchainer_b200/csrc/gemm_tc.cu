@@ -169,6 +169,11 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned pari
         }
     }
 }
+// the same for a whole warp in step: every lane tests, the outcome is the warp's
+__device__ __forceinline__ bool mbar_wait_warp(unsigned long long *bar, unsigned parity, volatile int *abort_flag, unsigned int *err) {
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, err));
+}
 
 // Bounded wait until the counter at `flag` (written by other CTAs of this launch) has reached `want`.
 __device__ __forceinline__ bool flag_wait(const unsigned *flag, unsigned want, volatile int *abort_flag, unsigned int *err) {
@@ -266,30 +271,42 @@ __device__ __forceinline__ void tc_mma_pair(unsigned tmem_d, unsigned long long 
                  : "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
-// forms for the MMA issue loop: descriptors as (low, high) words, barriers as shared-space addresses
+// Forms for the MMA issue loop, which a whole warp runs in step with one elected lane issuing: descriptors as (low, high) words,
+// barriers as shared-space addresses, `lead` the election's result.  The election is a predicate of the instruction, not a
+// branch around it: descriptors and TMEM addresses of an MMA live in uniform registers, and inside a one-lane branch the
+// compiler has to move each of them there from an ordinary register in front of every MMA (about 125 cycles per MMA, whatever
+// its size; a 128 x 128 x 16 one takes 64).
 template <bool PAIR>
 __device__ __forceinline__ void tc_mma_words(unsigned tmem_d, unsigned a_lo, unsigned a_hi, unsigned b_lo, unsigned b_hi, unsigned idesc,
-                                             unsigned accumulate) {
+                                             unsigned accumulate, unsigned lead) {
     if (PAIR)
-        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-                     "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}"
+        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+                     "@q tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}"
                      :
-                     : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+                     : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(lead)
                      : "memory");
     else
-        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
-                     "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
+        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\tmov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"
+                     "@q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n\t}"
                      :
-                     : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+                     : "r"(tmem_d), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(lead)
                      : "memory");
 }
-template <bool PAIR> __device__ __forceinline__ void tc_commit_addr(unsigned bar_addr) {
+template <bool PAIR> __device__ __forceinline__ void tc_commit_addr(unsigned bar_addr, unsigned lead) {
     if (PAIR)
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar_addr),
-                     "h"((unsigned short)3)
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t"
+                     "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar_addr),
+                     "h"((unsigned short)3), "r"(lead)
                      : "memory");
     else
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_addr) : "memory");
+        asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar_addr),
+                     "r"(lead)
+                     : "memory");
+}
+__device__ __forceinline__ unsigned elect_lane() {
+    unsigned e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e;
 }
 __device__ __forceinline__ bool mbar_test_addr(unsigned bar_addr, unsigned parity) {
     unsigned ok;
@@ -443,7 +460,8 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     unsigned *tmem_slot = (unsigned *)(acc_empty + 2);
     volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
 
-    int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // the warp index as a value the compiler knows to be the same in all lanes: what a role computes from it may stay uniform
+    const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
     // rank inside the pair (0 = leader: arms the full barriers and issues the MMAs) and the
     // persistent work stride: one work item per CTA, or per pair
     const unsigned crank = PAIR ? cluster_rank() : 0u;
@@ -478,7 +496,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     __syncthreads();
     if (PAIR) cluster_sync_all(); // the peer's barriers exist before anything signals them
     tc_fence_after();
-    unsigned tmem_base = *tmem_slot;
+    const unsigned tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     // everything above touched only shared and tensor memory, so it may run while the previous kernel of the
     // stream drains; from here on global memory is read and written
     dep_wait();
@@ -557,13 +575,15 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer (the leader, in a pair)
-        if (lane == 0 && crank == 0) {
-            // This thread's instruction stream is the critical path: every instruction between two
+        if (crank == 0) {
+            // This warp's instruction stream is the critical path: every instruction between two
             // MMAs costs a few cycles of tensor-pipe idle time.  So the loop carries ready-made
-            // descriptor words and barrier addresses and only adds small offsets to them.
+            // descriptor words and barrier addresses and only adds small offsets to them; all lanes
+            // run it (waits included), one elected lane issues.
+            const unsigned lead = elect_lane();
             unsigned tile_it = 0;
-            unsigned a_lbo = args.a_mn ? 8192u : 16u, a_kinc = (args.a_mn ? 2048u : 32u) >> 4;
-            unsigned b_lbo = args.b_mn ? 8192u : 16u, b_kinc = (args.b_mn ? 2048u : 32u) >> 4;
+            const unsigned a_lbo = args.a_mn ? 8192u : 16u, a_kinc = (args.a_mn ? 2048u : 32u) >> 4;
+            const unsigned b_lbo = args.b_mn ? 8192u : 16u, b_kinc = (args.b_mn ? 2048u : 32u) >> 4;
             const unsigned long long a_desc0 = make_desc(smem_u32(tiles), a_lbo, 1024u);
             const unsigned long long b_desc0 = make_desc(smem_u32(tiles) + kABytes, b_lbo, 1024u);
             // only the 14-bit start-address field changes (operands sit below 256 KB, so no carry)
@@ -579,24 +599,20 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 const int nkb = wi.kb1 - wi.kb0;
                 int acc = tile_it & 1;
                 unsigned acc_ph = (tile_it >> 1) & 1u;
-                if (!mbar_wait(&acc_empty[acc], acc_ph ^ 1u, abort_flag, args.err)) break;
+                if (!mbar_wait_warp(&acc_empty[acc], acc_ph ^ 1u, abort_flag, args.err)) break;
                 tc_fence_after();
                 const unsigned tmem_d = tmem_base + (unsigned)(acc * BN);
                 unsigned accum = 0; // the first MMA of a tile overwrites the accumulator
                 for (int i = 0; i < nkb; ++i) {
-                    if (!mbar_test_addr(full0 + s * 8u, ph)) {
-                        ok = mbar_wait(&full_bar[s], ph, abort_flag, args.err);
-                        if (!ok) break;
-                    }
+                    ok = mbar_wait_warp(&full_bar[s], ph, abort_flag, args.err);
+                    if (!ok) break;
                     const unsigned al = a_lo0 + soff, bl = b_lo0 + soff;
 #pragma unroll
-                    for (int j = 0; j < BK / 16; ++j) {
-                        if (PAIR) tc_mma_words<true>(tmem_d, al + j * a_kinc, a_hi, bl + j * b_kinc, b_hi, idesc, j == 0 ? accum : 1u);
-                        else tc_mma_words<false>(tmem_d, al + j * a_kinc, a_hi, bl + j * b_kinc, b_hi, idesc, j == 0 ? accum : 1u);
-                    }
+                    for (int j = 0; j < BK / 16; ++j)
+                        tc_mma_words<PAIR>(tmem_d, al + j * a_kinc, a_hi, bl + j * b_kinc, b_hi, idesc, j == 0 ? accum : 1u, lead);
                     accum = 1u;
                     // frees the smem stage (in both CTAs of a pair) once these MMAs have read it
-                    tc_commit_addr<PAIR>(empty0 + s * 8u);
+                    tc_commit_addr<PAIR>(empty0 + s * 8u, lead);
                     if (++s == nst) {
                         s = 0;
                         soff = 0;
@@ -607,7 +623,7 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
                 }
                 if (!ok) break;
                 // accumulator complete
-                tc_commit_addr<PAIR>(smem_u32(&acc_full[acc]));
+                tc_commit_addr<PAIR>(smem_u32(&acc_full[acc]), lead);
             }
         }
     } else {
