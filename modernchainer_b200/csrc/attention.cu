@@ -15,6 +15,8 @@ namespace {
 // in-place: row <- softmax(scale * row) over unmasked keys; masked entries become exactly 0.
 // lse (optional) receives max + log(sum) of the scaled scores.
 __global__ void attn_softmax_kernel(float *__restrict__ p, float *__restrict__ lse, int seq, float scale, int causal) {
+    dep_wait();
+    dep_trigger();
     __shared__ float red[32];
     long long row = blockIdx.x; // (n*heads + h)*seq + q
     int q = (int)(row % seq);
@@ -32,6 +34,8 @@ __global__ void attn_softmax_kernel(float *__restrict__ p, float *__restrict__ l
 
 // in-place on dp: ds = p * (dp - sum_k p*dp)
 __global__ void attn_dsoftmax_kernel(const float *__restrict__ p, float *__restrict__ dp, int seq) {
+    dep_wait();
+    dep_trigger();
     __shared__ float red[32];
     long long row = blockIdx.x;
     const float *pr = p + row * seq;
@@ -93,7 +97,7 @@ mcb_status probs(mcb_ctx *ctx, const float *q, const float *k, float *P, float *
     MCB_TRY(mcb_sgemm(ctx, p));
     float scale = 1.0f / sqrtf((float)hd);
     int threads = seq >= 512 ? 256 : (seq >= 64 ? 64 : 32);
-    attn_softmax_kernel<<<(unsigned)(n * heads * seq), threads, 0, ctx->stream>>>(P, lse, (int)seq, scale, causal);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, attn_softmax_kernel, dim3((unsigned)(n * heads * seq)), dim3(threads), 0, P, lse, (int)seq, scale, causal));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -197,7 +201,7 @@ mcb_status mcb_attention_backward(mcb_ctx *ctx, const void *q, const void *k, co
     p.a_bo = pb_o; p.a_bi = pb_i; p.b_bo = xb_o; p.b_bi = xb_i; p.c_bo = xb_o; p.c_bi = xb_i;
     MCB_TRY(mcb_sgemm(ctx, p));
     int threads = seq >= 512 ? 256 : (seq >= 64 ? 64 : 32);
-    attn_dsoftmax_kernel<<<(unsigned)(n * heads * seq), threads, 0, ctx->stream>>>((const float *)P, (float *)dP, (int)seq);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, attn_dsoftmax_kernel, dim3((unsigned)(n * heads * seq)), dim3(threads), 0, (const float *)P, (float *)dP, (int)seq));
     MCB_LAUNCHED(ctx);
     // dQ[q,d] = scale * sum_k dS[q,k] K[k,d]
     p = head_gemm(n, heads, seq, dim);

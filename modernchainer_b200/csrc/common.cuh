@@ -156,7 +156,9 @@ static inline int mcb_grid_for(mcb_ctx *ctx, int64_t work_items, int per_block, 
 // arithmetic, barrier initialisation and shared/tensor-memory set-up may come before.  dep_wait() returns
 // once all preceding kernels have completed and their writes are visible, so the stream stays in order;
 // what overlaps is launch latency, the prologue and the tail of the previous grid.  Both calls are no-ops
-// in a kernel launched the ordinary way.
+// in a kernel launched the ordinary way.  A pointer that is read unconditionally right behind dep_wait() is not declared
+// const __restrict__: that would allow the compiler to move the load in front of the wait.
+// (Between two launches of a few microseconds the ordinary way leaves a gap of 2 to 3 us, this one of about 1.)
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -223,6 +225,15 @@ __device__ __forceinline__ float warp_max(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     return v;
+}
+// sum of p[0..n) by one warp, the same order every time: lane l adds l, l + 32, ..., then a tree over the lanes
+__device__ __forceinline__ double warp_sum_f64(const double *p, int n) {
+    double t = 0.0;
+#pragma unroll 4
+    for (int i = threadIdx.x & 31; i < n; i += 32) t += p[i];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
 }
 // block-wide sum; `red` is shared float[32]; every thread gets the result
 __device__ __forceinline__ float block_sum(float v, float *red) {

@@ -27,6 +27,8 @@ template <int OP> __device__ __forceinline__ float bin_op(float x, float y) {
 template <int OP>
 __global__ void binary_fast_kernel(const float *__restrict__ a, const float *__restrict__ b, float *__restrict__ out,
                                    long long n, long long cols, int mode) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     if (mode == 0 && (n & 3) == 0) {
@@ -57,6 +59,8 @@ __global__ void binary_fast_kernel(const float *__restrict__ a, const float *__r
 template <int OP>
 __global__ void binary_generic_kernel(const float *__restrict__ a, const float *__restrict__ b,
                                       float *__restrict__ out, long long n, BinDims d) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (; i < n; i += stride) {
@@ -72,6 +76,8 @@ __global__ void binary_generic_kernel(const float *__restrict__ a, const float *
 }
 
 template <typename T> __global__ void add_inplace_kernel(T *__restrict__ dst, const T *__restrict__ src, long long n, int vec) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     long long n4 = vec ? (n >> 2) : 0;
@@ -83,6 +89,8 @@ template <typename T> __global__ void add_inplace_kernel(T *__restrict__ dst, co
 }
 
 __global__ void scale_kernel(const float *__restrict__ x, float f, float *__restrict__ out, long long n, int vec) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     long long n4 = vec ? (n >> 2) : 0;
@@ -94,12 +102,16 @@ __global__ void scale_kernel(const float *__restrict__ x, float f, float *__rest
 }
 
 __global__ void fill_kernel(float *__restrict__ out, float v, long long n) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (; i < n; i += stride) out[i] = v;
 }
 
 __global__ void unary_kernel(int op, const float *__restrict__ x, float *__restrict__ out, long long n) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (; i < n; i += stride) {
@@ -164,6 +176,8 @@ struct GeluBLowp {
 };
 
 template <typename T, typename Fn> __global__ void map1_kernel(const T *__restrict__ x, T *__restrict__ out, long long n, int vec) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     long long n4 = vec ? (n >> 2) : 0;
@@ -176,6 +190,8 @@ template <typename T, typename Fn> __global__ void map1_kernel(const T *__restri
 
 template <typename T, typename Fn>
 __global__ void map2_kernel(const T *__restrict__ x, const T *__restrict__ g, T *__restrict__ out, long long n, int vec) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     long long n4 = vec ? (n >> 2) : 0;
@@ -195,16 +211,22 @@ template <> __device__ __forceinline__ float cast_one<__half, float>(__half v) {
 template <> __device__ __forceinline__ float cast_one<float, float>(float v) { return v; }
 
 template <typename S, typename D> __global__ void cast_kernel(const S *__restrict__ src, D *__restrict__ dst, long long n) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (; i < n; i += stride) dst[i] = cast_one<S, D>(src[i]);
 }
 template <typename T> __global__ void cast_f32_lp_vec_kernel(const float *__restrict__ src, T *__restrict__ dst, long long n4) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (; i < n4; i += stride) Elem<T>::st4(dst, i, reinterpret_cast<const float4 *>(src)[i]);
 }
 template <typename T> __global__ void cast_lp_f32_vec_kernel(const T *__restrict__ src, float *__restrict__ dst, long long n4) {
+    dep_wait();
+    dep_trigger();
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
     for (; i < n4; i += stride) reinterpret_cast<float4 *>(dst)[i] = Elem<T>::ld4(src, i);
@@ -217,11 +239,11 @@ mcb_status launch_map1(mcb_ctx *ctx, const void *x, void *out, int64_t n, int32_
     ProfScope prof(ctx, MCB_PROF_ELEMENTWISE, 0.0, (double)n * 2.0 * (mcb_is_lp(dt) ? 2.0 : 4.0));
     int grid = mcb_grid_for(ctx, (n + 3) / 4, kThreads);
     if (dt == MCB_F32)
-        map1_kernel<float, Fn><<<grid, kThreads, 0, ctx->stream>>>((const float *)x, (float *)out, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, map1_kernel<float, Fn>, dim3(grid), dim3(kThreads), 0, (const float *)x, (float *)out, n, vec));
     else if (dt == MCB_BF16)
-        map1_kernel<__nv_bfloat16, Fn><<<grid, kThreads, 0, ctx->stream>>>((const __nv_bfloat16 *)x, (__nv_bfloat16 *)out, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, map1_kernel<__nv_bfloat16, Fn>, dim3(grid), dim3(kThreads), 0, (const __nv_bfloat16 *)x, (__nv_bfloat16 *)out, n, vec));
     else if (dt == MCB_F16)
-        map1_kernel<__half, Fn><<<grid, kThreads, 0, ctx->stream>>>((const __half *)x, (__half *)out, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, map1_kernel<__half, Fn>, dim3(grid), dim3(kThreads), 0, (const __half *)x, (__half *)out, n, vec));
     else
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "activation supports f32, bf16 and f16 storage");
     MCB_LAUNCHED(ctx);
@@ -234,12 +256,12 @@ mcb_status launch_map2(mcb_ctx *ctx, const void *x, const void *g, void *out, in
     ProfScope prof(ctx, MCB_PROF_ELEMENTWISE, 0.0, (double)n * 3.0 * (mcb_is_lp(dt) ? 2.0 : 4.0));
     int grid = mcb_grid_for(ctx, (n + 3) / 4, kThreads);
     if (dt == MCB_F32)
-        map2_kernel<float, Fn><<<grid, kThreads, 0, ctx->stream>>>((const float *)x, (const float *)g, (float *)out, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, map2_kernel<float, Fn>, dim3(grid), dim3(kThreads), 0, (const float *)x, (const float *)g, (float *)out, n, vec));
     else if (dt == MCB_BF16)
-        map2_kernel<__nv_bfloat16, Fn><<<grid, kThreads, 0, ctx->stream>>>((const __nv_bfloat16 *)x, (const __nv_bfloat16 *)g,
-                                                                           (__nv_bfloat16 *)out, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, map2_kernel<__nv_bfloat16, Fn>, dim3(grid), dim3(kThreads), 0, (const __nv_bfloat16 *)x, (const __nv_bfloat16 *)g,
+                                                                           (__nv_bfloat16 *)out, n, vec));
     else if (dt == MCB_F16)
-        map2_kernel<__half, Fn><<<grid, kThreads, 0, ctx->stream>>>((const __half *)x, (const __half *)g, (__half *)out, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, map2_kernel<__half, Fn>, dim3(grid), dim3(kThreads), 0, (const __half *)x, (const __half *)g, (__half *)out, n, vec));
     else
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "activation backward supports f32, bf16 and f16 storage");
     MCB_LAUNCHED(ctx);
@@ -351,9 +373,9 @@ mcb_status launch_binary(mcb_ctx *ctx, const float *a, const int64_t *ad, int ar
     if (mode == 0 && !(mcb_aligned16(a) && mcb_aligned16(b) && mcb_aligned16(out))) mode = 1, cols = n; // scalar path
     int grid = mcb_grid_for(ctx, mode == 0 ? (n + 3) / 4 : n, kThreads);
     if (mode >= 0)
-        binary_fast_kernel<OP><<<grid, kThreads, 0, ctx->stream>>>(a, b, out, n, cols, mode);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, binary_fast_kernel<OP>, dim3(grid), dim3(kThreads), 0, a, b, out, n, cols, mode));
     else
-        binary_generic_kernel<OP><<<grid, kThreads, 0, ctx->stream>>>(a, b, out, n, d);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, binary_generic_kernel<OP>, dim3(grid), dim3(kThreads), 0, a, b, out, n, d));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -382,11 +404,11 @@ mcb_status mcb_add_inplace(mcb_ctx *ctx, void *dst, const void *src, int64_t n, 
     ProfScope prof(ctx, MCB_PROF_ELEMENTWISE, 0.0, (double)n * 3.0 * (mcb_is_lp(dt) ? 2.0 : 4.0));
     int grid = mcb_grid_for(ctx, (n + 3) / 4, kThreads);
     if (dt == MCB_F32)
-        add_inplace_kernel<float><<<grid, kThreads, 0, ctx->stream>>>((float *)dst, (const float *)src, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, add_inplace_kernel<float>, dim3(grid), dim3(kThreads), 0, (float *)dst, (const float *)src, n, vec));
     else if (dt == MCB_BF16)
-        add_inplace_kernel<__nv_bfloat16><<<grid, kThreads, 0, ctx->stream>>>((__nv_bfloat16 *)dst, (const __nv_bfloat16 *)src, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, add_inplace_kernel<__nv_bfloat16>, dim3(grid), dim3(kThreads), 0, (__nv_bfloat16 *)dst, (const __nv_bfloat16 *)src, n, vec));
     else if (dt == MCB_F16)
-        add_inplace_kernel<__half><<<grid, kThreads, 0, ctx->stream>>>((__half *)dst, (const __half *)src, n, vec);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, add_inplace_kernel<__half>, dim3(grid), dim3(kThreads), 0, (__half *)dst, (const __half *)src, n, vec));
     else
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "add_inplace supports f32, bf16 and f16");
     MCB_LAUNCHED(ctx);
@@ -396,7 +418,7 @@ mcb_status mcb_add_inplace(mcb_ctx *ctx, void *dst, const void *src, int64_t n, 
 mcb_status mcb_scale(mcb_ctx *ctx, const float *x, double factor, float *out, int64_t n) {
     MCB_CHECK_CTX(ctx);
     if (n == 0) return MCB_OK;
-    scale_kernel<<<mcb_grid_for(ctx, (n + 3) / 4, kThreads), kThreads, 0, ctx->stream>>>(x, (float)factor, out, n, mcb_aligned16(x) && mcb_aligned16(out));
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, scale_kernel, dim3(mcb_grid_for(ctx, (n + 3) / 4, kThreads)), dim3(kThreads), 0, x, (float)factor, out, n, mcb_aligned16(x) && mcb_aligned16(out)));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -404,7 +426,7 @@ mcb_status mcb_scale(mcb_ctx *ctx, const float *x, double factor, float *out, in
 mcb_status mcb_fill(mcb_ctx *ctx, float *out, float value, int64_t n) {
     MCB_CHECK_CTX(ctx);
     if (n == 0) return MCB_OK;
-    fill_kernel<<<mcb_grid_for(ctx, n, kThreads), kThreads, 0, ctx->stream>>>(out, value, n);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, fill_kernel, dim3(mcb_grid_for(ctx, n, kThreads)), dim3(kThreads), 0, out, value, n));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -413,7 +435,7 @@ mcb_status mcb_unary(mcb_ctx *ctx, int32_t op, const float *x, float *out, int64
     MCB_CHECK_CTX(ctx);
     if (op < MCB_EXP || op > MCB_NEG) return mcb_fail(ctx, MCB_INVALID_ARGUMENT, "unknown unary op %d", op);
     if (n == 0) return MCB_OK;
-    unary_kernel<<<mcb_grid_for(ctx, n, kThreads), kThreads, 0, ctx->stream>>>(op, x, out, n);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, unary_kernel, dim3(mcb_grid_for(ctx, n, kThreads)), dim3(kThreads), 0, op, x, out, n));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -443,26 +465,26 @@ mcb_status mcb_cast(mcb_ctx *ctx, const void *src, int32_t src_dt, void *dst, in
     bool vec = (n & 3) == 0 && mcb_aligned16(src) && mcb_aligned16(dst);
     if (src_dt == MCB_F32 && dst_dt == MCB_BF16) {
         if (vec)
-            cast_f32_lp_vec_kernel<__nv_bfloat16><<<mcb_grid_for(ctx, n / 4, kThreads), kThreads, 0, ctx->stream>>>((const float *)src, (__nv_bfloat16 *)dst, n / 4);
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_f32_lp_vec_kernel<__nv_bfloat16>, dim3(mcb_grid_for(ctx, n / 4, kThreads)), dim3(kThreads), 0, (const float *)src, (__nv_bfloat16 *)dst, n / 4));
         else
-            cast_kernel<float, __nv_bfloat16><<<grid, kThreads, 0, ctx->stream>>>((const float *)src, (__nv_bfloat16 *)dst, n);
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_kernel<float, __nv_bfloat16>, dim3(grid), dim3(kThreads), 0, (const float *)src, (__nv_bfloat16 *)dst, n));
     } else if (src_dt == MCB_BF16 && dst_dt == MCB_F32) {
         if (vec)
-            cast_lp_f32_vec_kernel<__nv_bfloat16><<<mcb_grid_for(ctx, n / 4, kThreads), kThreads, 0, ctx->stream>>>((const __nv_bfloat16 *)src, (float *)dst, n / 4);
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_lp_f32_vec_kernel<__nv_bfloat16>, dim3(mcb_grid_for(ctx, n / 4, kThreads)), dim3(kThreads), 0, (const __nv_bfloat16 *)src, (float *)dst, n / 4));
         else
-            cast_kernel<__nv_bfloat16, float><<<grid, kThreads, 0, ctx->stream>>>((const __nv_bfloat16 *)src, (float *)dst, n);
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_kernel<__nv_bfloat16, float>, dim3(grid), dim3(kThreads), 0, (const __nv_bfloat16 *)src, (float *)dst, n));
     } else if (src_dt == MCB_F32 && dst_dt == MCB_F16) {
         if (vec)
-            cast_f32_lp_vec_kernel<__half><<<mcb_grid_for(ctx, n / 4, kThreads), kThreads, 0, ctx->stream>>>((const float *)src, (__half *)dst, n / 4);
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_f32_lp_vec_kernel<__half>, dim3(mcb_grid_for(ctx, n / 4, kThreads)), dim3(kThreads), 0, (const float *)src, (__half *)dst, n / 4));
         else
-            cast_kernel<float, __half><<<grid, kThreads, 0, ctx->stream>>>((const float *)src, (__half *)dst, n);
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_kernel<float, __half>, dim3(grid), dim3(kThreads), 0, (const float *)src, (__half *)dst, n));
     } else if (src_dt == MCB_F16 && dst_dt == MCB_F32) {
         if (vec)
-            cast_lp_f32_vec_kernel<__half><<<mcb_grid_for(ctx, n / 4, kThreads), kThreads, 0, ctx->stream>>>((const __half *)src, (float *)dst, n / 4);
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_lp_f32_vec_kernel<__half>, dim3(mcb_grid_for(ctx, n / 4, kThreads)), dim3(kThreads), 0, (const __half *)src, (float *)dst, n / 4));
         else
-            cast_kernel<__half, float><<<grid, kThreads, 0, ctx->stream>>>((const __half *)src, (float *)dst, n);
+            MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_kernel<__half, float>, dim3(grid), dim3(kThreads), 0, (const __half *)src, (float *)dst, n));
     } else if (src_dt == MCB_F32 && dst_dt == MCB_F32) {
-        cast_kernel<float, float><<<grid, kThreads, 0, ctx->stream>>>((const float *)src, (float *)dst, n);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, cast_kernel<float, float>, dim3(grid), dim3(kThreads), 0, (const float *)src, (float *)dst, n));
     } else {
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "cast %d -> %d is not supported", src_dt, dst_dt);
     }
@@ -473,7 +495,9 @@ mcb_status mcb_cast(mcb_ctx *ctx, const void *src, int32_t src_dt, void *dst, in
 } // extern "C"
 
 namespace {
-__global__ void fill_from_scalar_kernel(float *__restrict__ out, const float *__restrict__ scalar, double factor, long long n) {
+__global__ void fill_from_scalar_kernel(float *out, const float *scalar, double factor, long long n) {
+    dep_wait();
+    dep_trigger();
     // product in f64, then narrowed (Ops::full_like_scalar, crates/modern-chainer-core/src/storage.rs:337-345)
     float v = (float)((double)scalar[0] * factor);
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -481,7 +505,9 @@ __global__ void fill_from_scalar_kernel(float *__restrict__ out, const float *__
     for (; i < n; i += stride) out[i] = v;
 }
 template <typename T>
-__global__ void mul_scalar_ptr_kernel(const T *__restrict__ x, const float *__restrict__ scalar, T *__restrict__ out, long long n) {
+__global__ void mul_scalar_ptr_kernel(const T *x, const float *scalar, T *out, long long n) {
+    dep_wait();
+    dep_trigger();
     float f = scalar[0];
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
@@ -510,7 +536,7 @@ void launch_add_typed(mcb_ctx *ctx, const void *a, const void *b, void *out, lon
 
 mcb_status mcb_fill_from_scalar(mcb_ctx *ctx, float *out, const float *scalar, double factor, int64_t n) {
     if (n == 0) return MCB_OK;
-    fill_from_scalar_kernel<<<mcb_grid_for(ctx, n, kThreads), kThreads, 0, ctx->stream>>>(out, scalar, factor, n);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, fill_from_scalar_kernel, dim3(mcb_grid_for(ctx, n, kThreads)), dim3(kThreads), 0, out, scalar, factor, n));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -519,11 +545,11 @@ mcb_status mcb_mul_scalar_ptr(mcb_ctx *ctx, const void *x, const float *scalar, 
     if (n == 0) return MCB_OK;
     int grid = mcb_grid_for(ctx, n, kThreads);
     if (dt == MCB_F32)
-        mul_scalar_ptr_kernel<float><<<grid, kThreads, 0, ctx->stream>>>((const float *)x, scalar, (float *)out, n);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, mul_scalar_ptr_kernel<float>, dim3(grid), dim3(kThreads), 0, (const float *)x, scalar, (float *)out, n));
     else if (dt == MCB_BF16)
-        mul_scalar_ptr_kernel<__nv_bfloat16><<<grid, kThreads, 0, ctx->stream>>>((const __nv_bfloat16 *)x, scalar, (__nv_bfloat16 *)out, n);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, mul_scalar_ptr_kernel<__nv_bfloat16>, dim3(grid), dim3(kThreads), 0, (const __nv_bfloat16 *)x, scalar, (__nv_bfloat16 *)out, n));
     else if (dt == MCB_F16)
-        mul_scalar_ptr_kernel<__half><<<grid, kThreads, 0, ctx->stream>>>((const __half *)x, scalar, (__half *)out, n);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, mul_scalar_ptr_kernel<__half>, dim3(grid), dim3(kThreads), 0, (const __half *)x, scalar, (__half *)out, n));
     else
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "scalar multiply supports f32, bf16 and f16");
     MCB_LAUNCHED(ctx);

@@ -274,12 +274,14 @@ void launch_opt(mcb_ctx *ctx, int kind, int grid, float *p, const GT *g, float *
     else sgd_flat_kernel<GT, MCB_OPT_MOMENTUM_SGD><<<grid, kThreads, 0, s>>>(p, g, m, sh, n, k, inv_scale_dev, skip, step_dev, vec);
 }
 __global__ void increment_i32_kernel(int *p) {
+    dep_wait();
+    dep_trigger();
     if (threadIdx.x == 0 && blockIdx.x == 0) p[0] += 1;
 }
 } // namespace
 
 mcb_status mcb_increment_i32(mcb_ctx *ctx, int32_t *counter) {
-    increment_i32_kernel<<<1, 32, 0, ctx->stream>>>(counter);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, increment_i32_kernel, dim3(1), dim3(32), 0, counter));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -341,14 +343,17 @@ __global__ void sumsq_partial_kernel(const float *__restrict__ g, long long n, d
 // mean the optimizer will use (1 / world; 1 on a single rank): the limit applies to the mean, and the factor
 // max_norm / norm scales the sum and the mean alike.
 __global__ void clip_final_kernel(const double *__restrict__ partial, int count, double max_norm, double mean_factor, double *__restrict__ out) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double t = 0.0;
-    for (int i = 0; i < count; ++i) t += partial[i];
+    dep_wait();
+    dep_trigger();
+    const double t = warp_sum_f64(partial, count);
+    if (threadIdx.x != 0) return;
     double norm = sqrt(t) * mean_factor;
     out[0] = norm;
     out[1] = (norm > max_norm && norm > 0.0) ? max_norm / norm : 1.0;
 }
-__global__ void scale_by_clip_kernel(float *__restrict__ g, long long n, const double *__restrict__ clip) {
+__global__ void scale_by_clip_kernel(float *g, long long n, const double *clip) {
+    dep_wait();
+    dep_trigger();
     double f = clip[1];
     if (f == 1.0) return; // within the limit: gradients stay untouched (no pass over memory)
     float ff = (float)f;  // Ops::scale narrows the factor to f32 first
@@ -366,14 +371,14 @@ mcb_status mcb_sumsq_partial(mcb_ctx *ctx, const float *g, int64_t n, double *pa
     return MCB_OK;
 }
 mcb_status mcb_clip_finalize(mcb_ctx *ctx, const double *partial, int count, double max_norm, double *out2, double mean_factor) {
-    clip_final_kernel<<<1, 32, 0, ctx->stream>>>(partial, count, max_norm, mean_factor, out2);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, clip_final_kernel, dim3(1), dim3(32), 0, partial, count, max_norm, mean_factor, out2));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
 mcb_status mcb_scale_by_clip(mcb_ctx *ctx, float *g, int64_t n, const double *clip2) {
     if (n == 0) return MCB_OK;
     ProfScope prof(ctx, MCB_PROF_OPTIMIZER, 0.0, 8.0 * (double)n);
-    scale_by_clip_kernel<<<mcb_grid_for(ctx, n, kThreads, 8), kThreads, 0, ctx->stream>>>(g, n, clip2);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, scale_by_clip_kernel, dim3(mcb_grid_for(ctx, n, kThreads, 8)), dim3(kThreads), 0, g, n, clip2));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -381,6 +386,8 @@ mcb_status mcb_scale_by_clip(mcb_ctx *ctx, float *g, int64_t n, const double *cl
 namespace {
 // GradScaler::step bookkeeping (crates/modern-chainer-optim/src/amp.rs:66-86) on the device
 __global__ void scaler_update_kernel(float *sf, int *si, float growth, float backoff, int interval) {
+    dep_wait();
+    dep_trigger();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     int found = si[1];
     si[2] = found;
@@ -401,7 +408,7 @@ __global__ void scaler_update_kernel(float *sf, int *si, float growth, float bac
 } // namespace
 
 mcb_status mcb_scaler_update(mcb_ctx *ctx, float *state_f, int *state_i, float growth, float backoff, int interval) {
-    scaler_update_kernel<<<1, 32, 0, ctx->stream>>>(state_f, state_i, growth, backoff, interval);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, scaler_update_kernel, dim3(1), dim3(32), 0, state_f, state_i, growth, backoff, interval));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }

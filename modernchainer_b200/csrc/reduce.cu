@@ -14,6 +14,8 @@ constexpr int kThreads = 256;
 
 // ------------------------------------------------------------------ sum_all
 __global__ void sum_partial_kernel(const float *__restrict__ x, long long n, double *__restrict__ partial) {
+    dep_wait();
+    dep_trigger();
     __shared__ double red[kThreads / 32];
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
@@ -38,19 +40,21 @@ __global__ void sum_partial_kernel(const float *__restrict__ x, long long n, dou
         partial[blockIdx.x] = t;
     }
 }
-// out = (float)(scale * sum(partial[0..m))) in fixed order
+// out = (float)(scale * sum(partial[0..m))) in fixed order, by one warp.  One thread adding 592 partial sums took 14 us: a chain of
+// dependent loads and f64 adds; 32 interleaved chains and a tree take 2 us.
 __global__ void sum_final_kernel(const double *__restrict__ partial, int m, double scale, float *__restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double t = 0.0;
-        for (int i = 0; i < m; ++i) t += partial[i];
-        out[0] = (float)(t * scale);
-    }
+    dep_wait();
+    dep_trigger();
+    const double t = warp_sum_f64(partial, m);
+    if (threadIdx.x == 0) out[0] = (float)(t * scale);
 }
 
 // ------------------------------------------------------------------ column sums
 // grid (ceil(cols/32), splits), block (32, 8).  partial[split][col].
 template <typename T>
 __global__ void col_sum_partial_kernel(const T *__restrict__ a, long long rows, long long cols, float *__restrict__ partial) {
+    dep_wait();
+    dep_trigger();
     __shared__ float tile[8][33];
     long long col = (long long)blockIdx.x * 32 + threadIdx.x;
     long long rows_per = (rows + gridDim.y - 1) / gridDim.y;
@@ -126,6 +130,8 @@ __global__ void partial_sum_final_kernel(const float *__restrict__ partial, int 
     }
 }
 __global__ void col_sum_final_kernel(const float *__restrict__ partial, int splits, long long cols, float *__restrict__ out) {
+    dep_wait();
+    dep_trigger();
     long long col = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= cols) return;
     float t = 0.0f;
@@ -482,8 +488,10 @@ __device__ __forceinline__ void row_max_sumexp(const T *__restrict__ row, long l
     mx_out = M;
 }
 
-__global__ void sce_rows_kernel(const float *__restrict__ x, const void *__restrict__ labels, int label_dt,
+__global__ void sce_rows_kernel(const float *__restrict__ x, const void *labels, int label_dt,
                                 long long c, float *__restrict__ row_loss, unsigned int *err) {
+    dep_wait();
+    dep_trigger();
     __shared__ float red[32];
     long long i = blockIdx.x;
     long long lab = load_index(labels, label_dt, i);
@@ -500,6 +508,8 @@ __global__ void sce_rows_kernel(const float *__restrict__ x, const void *__restr
     if (threadIdx.x == 0) row_loss[i] = (mx + logf(sum)) - row[lab];
 }
 __global__ void sce_final_kernel(const float *__restrict__ row_loss, long long n, float *__restrict__ loss) {
+    dep_wait();
+    dep_trigger();
     __shared__ double red[kThreads];
     double acc = 0.0;
     for (long long i = threadIdx.x; i < n; i += blockDim.x) acc += (double)row_loss[i];
@@ -516,9 +526,11 @@ __global__ void sce_final_kernel(const float *__restrict__ row_loss, long long n
 // `stats_out` / `stats_in` ([n][2]: row maximum, sum of exp): the loss pass of a training step leaves them for the
 // gradient pass, which then needs no reduction over the row and streams it once.
 template <typename T>
-__global__ void __launch_bounds__(512, 3) sce_fused_kernel(const T *x, T *out, const void *__restrict__ labels, int label_dt, long long n,
-                                 long long c, float *__restrict__ row_loss, const float *__restrict__ upstream,
-                                 unsigned int *err, float *__restrict__ stats_out, const float *__restrict__ stats_in, long long ld) {
+__global__ void __launch_bounds__(512, 3) sce_fused_kernel(const T *x, T *out, const void *labels, int label_dt, long long n,
+                                 long long c, float *__restrict__ row_loss, const float *upstream,
+                                 unsigned int *err, float *__restrict__ stats_out, const float *stats_in, long long ld) {
+    dep_wait();
+    dep_trigger();
     __shared__ float red[32];
     long long i = blockIdx.x;
     long long lab = load_index(labels, label_dt, i);
@@ -609,9 +621,9 @@ __global__ void __launch_bounds__(512, 3) sce_fused_kernel(const T *x, T *out, c
 // use).  g = (softmax - onehot) * up / n with the softmax as one FMA and one ex2 per logit:
 // p = 2^(v * log2e - (mx * log2e + log2(sum))).  `out` may alias `x`: a chunk is written by the thread that read it.
 template <typename T>
-__global__ void __launch_bounds__(256) sce_grad_stream_kernel(const uint4 *x, uint4 *out, const void *__restrict__ labels, int label_dt,
-                                                              long long n, long long c, long long c8, const float *__restrict__ stats,
-                                                              const float *__restrict__ upstream, unsigned int *err) {
+__global__ void __launch_bounds__(256) sce_grad_stream_kernel(const uint4 *x, uint4 *out, const void *labels, int label_dt,
+                                                              long long n, long long c, long long c8, const float *stats,
+                                                              const float *upstream, unsigned int *err) {
     const long long row = blockIdx.y;
     const long long j0 = (long long)blockIdx.x * 1024 + threadIdx.x;
     const uint4 *r8 = x + row * c8;
@@ -658,6 +670,8 @@ __global__ void __launch_bounds__(256) sce_grad_stream_kernel(const uint4 *x, ui
 // ------------------------------------------------------------------ embedding
 __global__ void embedding_kernel(const void *__restrict__ ids, int id_dt, long long n, const float *__restrict__ w,
                                  long long vocab, int dim, float *__restrict__ out, unsigned int *err, int vec) {
+    dep_wait();
+    dep_trigger();
     int per_row = vec ? (dim >> 2) : dim;
     long long total = n * per_row;
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -680,6 +694,8 @@ template <typename GT>
 __global__ void embedding_backward_kernel(const void *__restrict__ ids, int id_dt, long long n,
                                           const GT *__restrict__ g, long long vocab, int dim, float *__restrict__ out,
                                           unsigned int *err) {
+    dep_wait();
+    dep_trigger();
     long long total = n * dim;
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     long long stride = (long long)gridDim.x * blockDim.x;
@@ -775,9 +791,9 @@ mcb_status mcb_sum_all(mcb_ctx *ctx, const float *x, int64_t n, float *out) {
     int grid = mcb_grid_for(ctx, n, kThreads, 4);
     void *scratch;
     MCB_TRY(mcb_scratch(ctx, sizeof(double) * grid, &scratch));
-    sum_partial_kernel<<<grid, kThreads, 0, ctx->stream>>>(x, n, (double *)scratch);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, sum_partial_kernel, dim3(grid), dim3(kThreads), 0, x, n, (double *)scratch));
     MCB_LAUNCHED(ctx);
-    sum_final_kernel<<<1, 32, 0, ctx->stream>>>((const double *)scratch, grid, 1.0, out);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, sum_final_kernel, dim3(1), dim3(32), 0, (const double *)scratch, grid, 1.0, out));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -818,15 +834,15 @@ mcb_status mcb_col_sum(mcb_ctx *ctx, const void *a, int32_t dt, int64_t rows, in
     MCB_TRY(mcb_scratch(ctx, sizeof(float) * splits * cols, &scratch));
     dim3 grid(col_tiles, splits), block(32, 8);
     if (dt == MCB_F32)
-        col_sum_partial_kernel<float><<<grid, block, 0, ctx->stream>>>((const float *)a, rows, cols, (float *)scratch);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, col_sum_partial_kernel<float>, dim3(grid), dim3(block), 0, (const float *)a, rows, cols, (float *)scratch));
     else if (dt == MCB_BF16)
-        col_sum_partial_kernel<__nv_bfloat16><<<grid, block, 0, ctx->stream>>>((const __nv_bfloat16 *)a, rows, cols, (float *)scratch);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, col_sum_partial_kernel<__nv_bfloat16>, dim3(grid), dim3(block), 0, (const __nv_bfloat16 *)a, rows, cols, (float *)scratch));
     else if (dt == MCB_F16)
-        col_sum_partial_kernel<__half><<<grid, block, 0, ctx->stream>>>((const __half *)a, rows, cols, (float *)scratch);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, col_sum_partial_kernel<__half>, dim3(grid), dim3(block), 0, (const __half *)a, rows, cols, (float *)scratch));
     else
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "col_sum supports f32, bf16 and f16");
     MCB_LAUNCHED(ctx);
-    col_sum_final_kernel<<<(int)((cols + 255) / 256), 256, 0, ctx->stream>>>((const float *)scratch, splits, cols, out);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, col_sum_final_kernel, dim3((int)((cols + 255) / 256)), dim3(256), 0, (const float *)scratch, splits, cols, out));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -976,9 +992,9 @@ mcb_status mcb_softmax_cross_entropy(mcb_ctx *ctx, const float *logits, const vo
     void *scratch;
     MCB_TRY(mcb_scratch(ctx, sizeof(float) * n, &scratch));
     int threads = c >= 4096 ? 512 : (c >= 256 ? 128 : 32);
-    sce_rows_kernel<<<(unsigned)n, threads, 0, ctx->stream>>>(logits, labels, label_dt, c, (float *)scratch, ctx->d_err);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, sce_rows_kernel, dim3((unsigned)n), dim3(threads), 0, logits, labels, label_dt, c, (float *)scratch, ctx->d_err));
     MCB_LAUNCHED(ctx);
-    sce_final_kernel<<<1, kThreads, 0, ctx->stream>>>((const float *)scratch, n, loss_out);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, sce_final_kernel, dim3(1), dim3(kThreads), 0, (const float *)scratch, n, loss_out));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -1002,7 +1018,7 @@ mcb_status mcb_embedding(mcb_ctx *ctx, const void *ids, int32_t id_dt, int64_t n
     if (n == 0 || dim == 0) return MCB_OK;
     int vec = (dim % 4 == 0) && mcb_aligned16(weight) && mcb_aligned16(out);
     long long total = n * (vec ? dim / 4 : dim);
-    embedding_kernel<<<mcb_grid_for(ctx, total, kThreads), kThreads, 0, ctx->stream>>>(ids, id_dt, n, weight, vocab, (int)dim, out, ctx->d_err, vec);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, embedding_kernel, dim3(mcb_grid_for(ctx, total, kThreads)), dim3(kThreads), 0, ids, id_dt, n, weight, vocab, (int)dim, out, ctx->d_err, vec));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
@@ -1029,11 +1045,11 @@ mcb_status mcb_embedding_backward(mcb_ctx *ctx, const void *ids, int32_t id_dt, 
     }
     int grid = mcb_grid_for(ctx, n * dim, kThreads);
     if (g_dt == MCB_F32)
-        embedding_backward_kernel<float><<<grid, kThreads, 0, ctx->stream>>>(ids, id_dt, n, (const float *)g, vocab, (int)dim, out, ctx->d_err);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, embedding_backward_kernel<float>, dim3(grid), dim3(kThreads), 0, ids, id_dt, n, (const float *)g, vocab, (int)dim, out, ctx->d_err));
     else if (g_dt == MCB_BF16)
-        embedding_backward_kernel<__nv_bfloat16><<<grid, kThreads, 0, ctx->stream>>>(ids, id_dt, n, (const __nv_bfloat16 *)g, vocab, (int)dim, out, ctx->d_err);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, embedding_backward_kernel<__nv_bfloat16>, dim3(grid), dim3(kThreads), 0, ids, id_dt, n, (const __nv_bfloat16 *)g, vocab, (int)dim, out, ctx->d_err));
     else if (g_dt == MCB_F16)
-        embedding_backward_kernel<__half><<<grid, kThreads, 0, ctx->stream>>>(ids, id_dt, n, (const __half *)g, vocab, (int)dim, out, ctx->d_err);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, embedding_backward_kernel<__half>, dim3(grid), dim3(kThreads), 0, ids, id_dt, n, (const __half *)g, vocab, (int)dim, out, ctx->d_err));
     else
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "embedding grad must be f32, bf16 or f16");
     MCB_LAUNCHED(ctx);
@@ -1069,16 +1085,16 @@ mcb_status mcb_sce_grad(mcb_ctx *ctx, const void *logits, void *out, int32_t dt,
         return MCB_OK;
     }
     if (dt == MCB_F32)
-        sce_fused_kernel<float><<<(unsigned)n, threads, 0, ctx->stream>>>((const float *)logits, (float *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, sce_fused_kernel<float>, dim3((unsigned)n), dim3(threads), 0, (const float *)logits, (float *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld));
     else if (dt == MCB_BF16)
-        sce_fused_kernel<__nv_bfloat16><<<(unsigned)n, threads, 0, ctx->stream>>>((const __nv_bfloat16 *)logits, (__nv_bfloat16 *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, sce_fused_kernel<__nv_bfloat16>, dim3((unsigned)n), dim3(threads), 0, (const __nv_bfloat16 *)logits, (__nv_bfloat16 *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld));
     else if (dt == MCB_F16)
-        sce_fused_kernel<__half><<<(unsigned)n, threads, 0, ctx->stream>>>((const __half *)logits, (__half *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, sce_fused_kernel<__half>, dim3((unsigned)n), dim3(threads), 0, (const __half *)logits, (__half *)out, labels, label_dt, n, c, (float *)scratch, upstream, ctx->d_err, stats_out, stats_in, ld));
     else
         return mcb_fail(ctx, MCB_UNSUPPORTED_DTYPE, "logits must be f32, bf16 or f16");
     MCB_LAUNCHED(ctx);
     if (loss_out) {
-        sce_final_kernel<<<1, kThreads, 0, ctx->stream>>>((const float *)scratch, n, loss_out);
+        MCB_CUDA(ctx, mcb_launch_dep(ctx, sce_final_kernel, dim3(1), dim3(kThreads), 0, (const float *)scratch, n, loss_out));
         MCB_LAUNCHED(ctx);
     }
     return MCB_OK;
@@ -1089,9 +1105,9 @@ mcb_status mcb_sum_scaled(mcb_ctx *ctx, const float *x, int64_t n, double scale,
     int grid = mcb_grid_for(ctx, n > 0 ? n : 1, kThreads, 4);
     void *scratch;
     MCB_TRY(mcb_scratch(ctx, sizeof(double) * grid, &scratch));
-    sum_partial_kernel<<<grid, kThreads, 0, ctx->stream>>>(x, n, (double *)scratch);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, sum_partial_kernel, dim3(grid), dim3(kThreads), 0, x, n, (double *)scratch));
     MCB_LAUNCHED(ctx);
-    sum_final_kernel<<<1, 32, 0, ctx->stream>>>((const double *)scratch, grid, scale, out);
+    MCB_CUDA(ctx, mcb_launch_dep(ctx, sum_final_kernel, dim3(1), dim3(32), 0, (const double *)scratch, grid, scale, out));
     MCB_LAUNCHED(ctx);
     return MCB_OK;
 }
