@@ -698,7 +698,7 @@ static mcb_status linear_backward_impl(mcb_ctx *ctx, const Tensor &g_in, const L
             pw.b = sv.x.ptr; pw.b_mn_major = 1; pw.ldb = k;
             pw.d = gi[1].ptr; pw.out_dt = MCB_F32; pw.ldd = k;
             pw.m = n; pw.n = k; pw.k = m;
-            mcb_tc_plan(ctx, n, k, m, true, false, 1, &pw.bn, &pw.split_k);
+            mcb_tc_plan(ctx, n, k, m, true, true, 1, &pw.bn, &pw.split_k);
             if (pw.split_k > 1) {
                 pw.accumulate = 1;
                 clear_dw = true;
@@ -1305,7 +1305,7 @@ mcb_status f_qkv_attention(const Var &x, const Var &wq, const Var &bq, const Var
         pw.b = xb.ptr; pw.b_mn_major = 1; pw.ldb = d;
         pw.d = dw.ptr; pw.out_dt = MCB_F32; pw.ldd = d;
         pw.m = 3 * d; pw.n = d; pw.k = m;
-        mcb_tc_plan(ctx, pw.m, pw.n, pw.k, true, false, 1, &pw.bn, &pw.split_k);
+        mcb_tc_plan(ctx, pw.m, pw.n, pw.k, true, true, 1, &pw.bn, &pw.split_k);
         bool clear_dw = false; // a split reduction adds its slices into a zero output: cleared by the GEMM in front where there is one
         if (pw.split_k > 1) {
             pw.accumulate = 1;

@@ -24,6 +24,7 @@
 // error word, stops issuing work, and still frees its TMEM before returning.
 #include <cuda.h>
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "common.cuh"
@@ -69,12 +70,7 @@ struct TcArgs {
     unsigned int *err;
 };
 
-constexpr int kFixTiles = 148;        // split-tail tiles a launch may finish in the kernel (size of mcb_ctx::tc_fix_cnt)
-// planner's charge for leaving and collecting the partial sums of a split tail.  Measured on 8192-row problems with 768
-// output columns (96 tiles of 256 x 256 on 74 CTA pairs): K = 3072 gains 2 us over 128 x 192 tiles, K = 2304 loses 2 us,
-// K = 768 loses 8 us; 7000 cycles puts the line between the first two.
-constexpr double kFixCycles = 7000.0;
-
+constexpr int kFixTiles = 148; // split-tail tiles a launch may finish in the kernel (size of mcb_ctx::tc_fix_cnt)
 struct WorkItem {
     unsigned t;   // tile index (tn-major: t = tn * m_tiles + tm)
     int kb0, kb1; // k-block range
@@ -201,6 +197,9 @@ __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *m
                  : "r"(smem_u32(smem_dst)), "l"((unsigned long long)map), "r"(smem_u32(bar)), "r"(x), "r"(y)
                  : "memory");
 }
+
+// fetches a tensor map (a kernel parameter) into the descriptor cache ahead of the first copy that uses it
+__device__ __forceinline__ void prefetch_map(const CUtensorMap *map) { asm volatile("prefetch.tensormap [%0];" ::"l"((unsigned long long)map) : "memory"); }
 
 __device__ __forceinline__ void tmem_alloc(unsigned *smem_dst, unsigned ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
@@ -428,14 +427,15 @@ __device__ __forceinline__ float gelu_f(float v) {
 template <int BN, bool PAIR> struct Cfg {
     static constexpr int kBRows = PAIR ? BN / 2 : BN; // B rows (output columns) staged per CTA
     static constexpr int kStageBytes = (BM + kBRows) * BK * 2;
-    static constexpr int kStages = PAIR ? (BN == 128 ? 8 : 6) : (BN == 128 ? 6 : 4);
+    static constexpr int kStages = PAIR ? 6 : (BN == 128 ? 6 : 4);
+    static_assert(!PAIR || BN == 256, "the pair form is built for 256-wide tiles");
     // Output boxes: 4 KB each, `ring` per epilogue warp.  One epilogue group (four warps, one per TMEM lane quarter) needs
     // 32 KB with two boxes each.  Tiles whose main loop is short (K of a few hundred) are bound by the epilogue, so where
     // shared memory allows a second group of four warps takes every other 64-column chunk: 128 x 192 tiles have the room
     // beside their four stages, 256-wide pair tiles give up one of six stages for it (chosen per launch).
-    static constexpr int kMaxGroups = ((BN == 192 && !PAIR) || (BN == 256 && PAIR)) ? 2 : 1;
+    static constexpr int kMaxGroups = (BN == 192 || PAIR) ? 2 : 1;
     static constexpr int kOutStageBytes = 4 * 2 * 4096;
-    static constexpr int kTileAndOutBytes = (BN == 256 && PAIR) ? (kStages * kStageBytes + kOutStageBytes) /* = 5 stages + 64 KB */
+    static constexpr int kTileAndOutBytes = PAIR ? (kStages * kStageBytes + kOutStageBytes) /* = 5 stages + 64 KB */
                                                                 : (kStages * kStageBytes + kMaxGroups * kOutStageBytes);
     static constexpr int kSmemBytes = kTileAndOutBytes + 1024 /*align*/ + 256 /*barriers*/;
     static_assert(kSmemBytes <= 227 * 1024, "shared memory budget of one CTA");
@@ -472,6 +472,10 @@ tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     constexpr int kTileM = PAIR ? 2 * BM : BM;
     const unsigned nst = (unsigned)args.stages; // ring depth in use, <= kStages
     if (threadIdx.x == 0) {
+        prefetch_map(&map_a);
+        prefetch_map(&map_b);
+        if (args.tma_out) prefetch_map(&map_d);
+        if (args.tma_out && args.d_pre) prefetch_map(&map_pre);
         for (int s = 0; s < kStages; ++s) {
             mbar_init(&full_bar[s], 2); // one arming arrival per operand producer
             mbar_init(&empty_bar[s], 1);
@@ -1032,12 +1036,12 @@ template <int BN, bool PAIR> mcb_status launch(mcb_ctx *ctx, const TcGemmParams 
     const bool one_group = knob_val(ctx, K_TC_EPI, 0) == 1;
     a.epi_groups = 1;
     const int short_kb = knob_val(ctx, K_TC_EPI_KB, 16); // tuning knob: k-blocks per item up to which the stage is traded
-    if (PAIR && BN == 256 && a.kb_per_split <= short_kb && C::kStageBytes * 1 >= 4 * 2 * 4096 && !knob_on(ctx, K_TC_STAGES)) {
+    if (PAIR && a.kb_per_split <= short_kb && C::kStageBytes * 1 >= 4 * 2 * 4096 && !knob_on(ctx, K_TC_STAGES)) {
         a.stages = C::kStages - 1;
         if (one_group) a.ring = 4;
         else a.epi_groups = 2;
     }
-    if (BN == 192 && !PAIR && !one_group) a.epi_groups = 2; // 128 x 192 tiles: room for both groups beside the four stages
+    if (BN == 192 && !one_group) a.epi_groups = 2; // 128 x 192 tiles: room for both groups beside the four stages
     if (knob_on(ctx, K_TC_STAGES)) {
         int v = knob_val(ctx, K_TC_STAGES, 0);
         if (v >= 2 && v < C::kStages) a.stages = v;
@@ -1119,7 +1123,7 @@ template <int BN, bool PAIR> mcb_status launch(mcb_ctx *ctx, const TcGemmParams 
     cudaError_t le;
     if (!PAIR) {
         int grid = (int)(work < ctx->sm_count ? work : ctx->sm_count);
-        le = mcb_launch_dep(ctx, tc_gemm_kernel<BN, false>, dim3(grid), dim3(kThreads), C::kSmemBytes, map_a, map_b, map_d, map_pre, a);
+        le = mcb_launch_dep(ctx, tc_gemm_kernel<BN, PAIR>, dim3(grid), dim3(kThreads), C::kSmemBytes, map_a, map_b, map_d, map_pre, a);
     } else {
         int pairs = (int)(work < max_pairs ? work : max_pairs);
         cudaLaunchConfig_t cfg = {};
@@ -1136,7 +1140,7 @@ template <int BN, bool PAIR> mcb_status launch(mcb_ctx *ctx, const TcGemmParams 
         at[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = at;
         cfg.numAttrs = ctx->dep_launch ? 2 : 1;
-        le = cudaLaunchKernelEx(&cfg, tc_gemm_kernel<BN, true>, map_a, map_b, map_d, map_pre, a);
+        le = cudaLaunchKernelEx(&cfg, tc_gemm_kernel<BN, PAIR>, map_a, map_b, map_d, map_pre, a);
     }
     if (ws) mcb_free(ctx, ws); // stream-ordered reuse: whoever gets the block next is enqueued behind this kernel
     MCB_CUDA(ctx, le);
@@ -1145,6 +1149,90 @@ template <int BN, bool PAIR> mcb_status launch(mcb_ctx *ctx, const TcGemmParams 
 }
 
 } // namespace
+
+namespace {
+// Time of one GEMM in microseconds, launch included, as a line fitted per tile form to 760 measured (shape, form, split) triples:
+// outputs of 128 .. 8192 rows by 256 .. 3072 columns, reductions of 256 .. 8192, forward (16-bit output) and weight gradient (f32
+// output, 1 to 16 slices), mean error 2%.  `kb` counts the k-blocks a worker walks, `kb_full` the same weighted by how full the
+// waves are (all SMs busy slow one another down), `wave` every wave behind the first, `f32` / `f32_wave` a 32-bit output, `add`
+// a million f32 outputs reduced into once, `kb_mn` a k-block of a data gradient (B stored with its columns contiguous arrives in
+// 64-column boxes, more of them per CTA in the single-CTA forms).
+// What the fit says: two CTAs on a 256-wide tile cost 1.3 us more at launch and exit and 0.07 us less per k-block, so they pay
+// from about 20 k-blocks per worker on; on 128-wide tiles they never pay (2048 x 256 x 256: 6.4 us against 5.1 for single CTAs).
+struct TcForm {
+    int bn, pair;
+    double base, kb, kb_full, wave, f32, f32_wave, add, kb_mn;
+};
+constexpr TcForm kForms[] = {{128, 0, 4.25, 0.193, 0.037, 0.51, 0.96, 0.85, 0.029, 0.040},
+                             {192, 0, 4.15, 0.259, 0.070, 0.27, 1.60, 1.43, 0.062, 0.035},
+                             {256, 0, 5.33, 0.319, 0.051, 0.64, 1.55, 1.91, 0.036, 0.052},
+                             {256, 1, 6.60, 0.297, 0.008, 1.18, 1.05, 0.51, 0.297, 0.020}};
+const TcForm &tc_form(int bn, int pair) {
+    for (const TcForm &f : kForms)
+        if (f.bn == bn && f.pair == pair) return f;
+    return kForms[0];
+}
+long long tc_tiles(const TcForm &f, long long m, long long n) {
+    const long long rows = f.pair ? 2 * BM : BM;
+    return ((m + rows - 1) / rows) * ((n + f.bn - 1) / f.bn);
+}
+double tc_cost(mcb_ctx *ctx, const TcForm &f, long long m, long long n, long long k, int split, bool f32_out, bool dgrad) {
+    const long long workers = f.pair ? ctx->sm_count / 2 : ctx->sm_count, kb_total = (k + BK - 1) / BK;
+    const long long kb = (kb_total + split - 1) / split, slices = (kb_total + kb - 1) / kb, items = tc_tiles(f, m, n) * slices;
+    const double waves = (double)((items + workers - 1) / workers);
+    return f.base + (f.kb + (dgrad ? f.kb_mn : 0.0)) * waves * (double)kb + f.kb_full * (double)items * (double)kb / (double)workers +
+           f.wave * (waves - 1.0) + (f32_out ? f.f32 + f.f32_wave * (waves - 1.0) : 0.0) +
+           (slices > 1 ? f.add * 1e-6 * (double)m * (double)n * (double)slices : 0.0);
+}
+// Slices of the tiles of a mostly empty last wave of 256 x 256 pair tiles (1: no such tail), and the time that form takes.
+// Leaving and collecting the slices' partial sums costs 3.7 us: 8192-row problems with 768 output columns (96 tiles on 74 CTA
+// pairs) gain 2 us over 128 x 192 tiles at K = 3072, lose 2 us at K = 2304 and 8 us at K = 768.  Slices that add straight
+// into an accumulating output cost 0.5 us.
+int tc_tail_slices(mcb_ctx *ctx, long long m, long long n, long long k) {
+    const long long workers = ctx->sm_count / 2, tiles = m <= BM ? 0 : tc_tiles(tc_form(256, 1), m, n);
+    if (tiles <= workers) return 1;
+    const long long rem = tiles % workers;
+    if (rem == 0) return 1;
+    return (int)std::max(1ll, std::min({workers / rem, 8ll, (k + BK - 1) / BK / 4}));
+}
+double tc_tail_cost(mcb_ctx *ctx, long long m, long long n, long long k, int slices, bool f32_out, bool dgrad, bool direct) {
+    const TcForm &f = tc_form(256, 1);
+    const long long workers = ctx->sm_count / 2, kb = (k + BK - 1) / BK, full = tc_tiles(f, m, n) / workers;
+    const double walked = (double)(full * kb + (kb + slices - 1) / slices);
+    return f.base + (f.kb + f.kb_full + (dgrad ? f.kb_mn : 0.0)) * walked + f.wave * (double)full +
+           (f32_out ? f.f32 + f.f32_wave * (double)full : 0.0) + (direct ? 0.5 : 3.7);
+}
+
+// Picks the tile width and, when the caller can zero the output and accept atomic accumulation, the split of the reduction:
+// the form that tc_cost (or tc_tail_cost) puts first.  Slices need an output that has been cleared, which costs about 1 us per
+// million values.
+void plan_form(mcb_ctx *ctx, long long m, long long n, long long k, bool allow_split, bool f32_out, bool dgrad, int fixed_split, int *bn_out,
+               int *split_out) {
+    const long long kb_total = (k + BK - 1) / BK;
+    double best = 0.0;
+    *bn_out = 0;
+    *split_out = 1;
+    for (const TcForm &f : kForms) {
+        if (f.pair && m <= BM) continue;
+        for (int s = 1; s <= (allow_split ? 16 : 1); ++s) {
+            const int split = allow_split ? s : std::max(fixed_split, 1);
+            if (split > 1 && kb_total / split < 4 && allow_split) break;
+            double t = tc_cost(ctx, f, m, n, k, split, f32_out, dgrad) + (allow_split && split > 1 ? 1.0e-6 * (double)m * (double)n : 0.0);
+            const int slices = f.pair && split == 1 ? tc_tail_slices(ctx, m, n, k) : 1;
+            if (slices > 1) t = std::min(t, tc_tail_cost(ctx, m, n, k, slices, f32_out, dgrad, false));
+            if (*bn_out == 0 || t < best) {
+                best = t;
+                *bn_out = f.bn;
+                *split_out = split;
+            }
+        }
+    }
+}
+} // namespace
+
+void mcb_tc_plan(mcb_ctx *ctx, int64_t m, int64_t n, int64_t k, bool allow_split, bool f32_out, int fixed_split, int *bn_out, int *split_out) {
+    plan_form(ctx, m, n, k, allow_split, f32_out, false, fixed_split, bn_out, split_out);
+}
 
 mcb_status mcb_tc_gemm(mcb_ctx *ctx, const TcGemmParams &p) {
     if (p.zero_ptr && (p.m == 0 || p.n == 0 || p.k == 0)) MCB_TRY(mcb_memset(ctx, p.zero_ptr, 0, p.zero_bytes)); // no kernel will run: clear it here
@@ -1166,6 +1254,7 @@ mcb_status mcb_tc_gemm(mcb_ctx *ctx, const TcGemmParams &p) {
     // vector stores in the epilogue need ldd and d aligned; otherwise the scalar tail path is used per row
     if ((mcb_is_lp(p.out_dt) && ((p.ldd % 8) || !mcb_aligned16(p.d))) || (p.out_dt == MCB_F32 && !p.accumulate && ((p.ldd % 4) || !mcb_aligned16(p.d))))
         return mcb_fail(ctx, MCB_INVALID_ARGUMENT, "GEMM output needs a 16-byte aligned base and row pitch");
+    const bool f32_out = p.out_dt == MCB_F32, dgrad = p.b_mn_major && !p.a_mn_major;
     int bn = p.bn, split = p.split_k < 1 ? 1 : p.split_k;
     // reproducible runs: slices of one reduction reach the output in arrival order, so there are none
     const bool fixed_order = knob_on(ctx, K_DETERMINISTIC);
@@ -1173,40 +1262,23 @@ mcb_status mcb_tc_gemm(mcb_ctx *ctx, const TcGemmParams &p) {
     bn = knob_val(ctx, K_TC_BN, bn); // tuning knob: force the tile width
     if (bn != 128 && bn != 192 && bn != 256) {
         int s2 = split;
-        mcb_tc_plan(ctx, p.m, p.n, p.k, false, p.accumulate, split, &bn, &s2);
+        plan_form(ctx, p.m, p.n, p.k, false, f32_out, dgrad, split, &bn, &s2);
     }
     TcGemmParams q = p;
     q.split_k = split;
     int pair = p.pair;
     pair = knob_val(ctx, K_TC_PAIR, pair); // tuning knob: 0 single CTA, 1 CTA pair
-    if (pair < 0) pair = (bn != 192 && p.m > 128) ? 1 : 0;
-    if (bn == 192) pair = 0; // half of 192 columns is not a whole number of 64-column boxes
-    // Split tail on 256 x 256 pair tiles against the planned form, by the same cycle estimate as mcb_tc_plan
-    // plus kFixCycles for leaving and collecting the partial sums of the slices
+    auto cost = [&](int w, int two) { return tc_cost(ctx, tc_form(w, two), p.m, p.n, p.k, split, f32_out, dgrad); };
+    if (bn != 256 || p.m <= BM) pair = 0;
+    if (pair < 0) pair = cost(256, 1) < cost(256, 0);
+    // Split tail on 256 x 256 pair tiles against the planned form
     int tail = p.split_tail;
     tail = knob_val(ctx, K_TC_SPLIT_TAIL, tail); // tuning knob: 0 never, 1 whenever it applies
     if (fixed_order && p.accumulate) tail = 0; // (a tail finished in the kernel adds in slice order: reproducible as it is)
     const bool tail_ok = (p.accumulate ? (p.bias == nullptr) : (split == 1)) && p.m > 128 && !knob_on(ctx, K_TC_BN);
     if (tail < 0 && tail_ok) {
-        const long long kb = (p.k + BK - 1) / BK, workers = ctx->sm_count / 2;
-        const long long tiles = ((p.m + 255) / 256) * ((p.n + 255) / 256), rem = tiles % workers;
-        long long s = rem > 0 ? workers / rem : 1;
-        if (s > 8) s = 8;
-        if (s > kb / 4) s = kb / 4;
-        tail = 0;
-        if (tiles > workers && s >= 2) {
-            const double per_tail = 4.0 * 128.0 + 60.0;
-            // an accumulating output takes the slices directly; otherwise workspace memset + finishing kernel
-            const double cost_tail = (double)((tiles / workers) * kb + (kb + s - 1) / s) * per_tail + 12.0 * 256 + (p.accumulate ? 1000.0 : kFixCycles);
-            // the planned form: `split` slices of every tile
-            const long long w_now = pair ? ctx->sm_count / 2 : ctx->sm_count;
-            const long long t_now = ((p.m + (pair ? 255 : 127)) / (pair ? 256 : 128)) * ((p.n + bn - 1) / bn);
-            const long long kb_item = (kb + split - 1) / split, items = t_now * ((kb + kb_item - 1) / kb_item);
-            const double mma = bn / 2.0 > 125.0 ? bn / 2.0 : 125.0;
-            const double cost_now = (double)((items + w_now - 1) / w_now) * (double)kb_item * (4.0 * mma + 60.0) + (p.accumulate ? 12.0 : 5.0) * bn +
-                                    (split > 1 ? 300.0 * split + (double)(split - 1) * (double)p.m * (double)p.n * 1.0e-3 : 0.0);
-            if (cost_tail < 0.9 * cost_now) tail = 1;
-        }
+        const int slices = tc_tail_slices(ctx, p.m, p.n, p.k);
+        tail = slices > 1 && tc_tail_cost(ctx, p.m, p.n, p.k, slices, f32_out, dgrad, p.accumulate != 0) < 0.95 * cost(bn, pair);
     }
     if (!tail_ok || tail < 0) tail = 0;
     q.split_tail = tail;
@@ -1215,66 +1287,10 @@ mcb_status mcb_tc_gemm(mcb_ctx *ctx, const TcGemmParams &p) {
         pair = 1;
         q.split_k = 1; // the tail is the only part that is cut along K
     }
-    if (pair) {
-        if (bn == 256) return launch<256, true>(ctx, q);
-        return launch<128, true>(ctx, q);
-    }
+    if (pair) return launch<256, true>(ctx, q);
     if (bn == 256) return launch<256, false>(ctx, q);
     if (bn == 192) return launch<192, false>(ctx, q);
     return launch<128, false>(ctx, q);
-}
-
-// Picks the tile width (and, when the caller can zero the output and accept atomic accumulation,
-// the split of the reduction dimension) that minimises a cycle estimate for one CTA:
-//   waves * k_blocks_per_item * (4 * max(BN/2, 125) + 60)  +  exposed epilogue
-// where the first term is the time of the four K=16 MMAs of one 64-deep block at M=128.
-void mcb_tc_plan(mcb_ctx *ctx, int64_t m, int64_t n, int64_t k, bool allow_split, bool atomic_out, int fixed_split, int *bn_out,
-                 int *split_out) {
-    const int cands[3] = {256, 192, 128};
-    long long m_tiles = (m + BM - 1) / BM, kb_total = (k + BK - 1) / BK;
-    double best = 1e300;
-    int best_bn = 256, best_split = 1;
-    int max_split = allow_split ? 16 : 1;
-    for (int i = 0; i < 3; ++i) {
-        int bn = cands[i];
-        long long tiles = m_tiles * ((n + bn - 1) / bn);
-        for (int s = 1; s <= max_split; ++s) {
-            int sp = allow_split ? s : (fixed_split < 1 ? 1 : fixed_split);
-            if (sp > 1 && kb_total / sp < 4) break;
-            long long kb = (kb_total + sp - 1) / sp;
-            long long items = tiles * ((kb_total + kb - 1) / kb);
-            long long waves = (items + ctx->sm_count - 1) / ctx->sm_count;
-            bool atomics = atomic_out || sp > 1;
-            double epi = (atomics ? 12.0 : 5.0) * bn;
-            // with several waves the epilogue of all but the last tile hides behind the next tile's MMAs
-            // one K=16 MMA at M=128 takes bn/2 cycles but never less than ~125 (the A operand's 4 KB
-            // leave shared memory at 32 B/clk), so narrow tiles run the tensor pipe below its rate
-            double mma = bn / 2.0 > 125.0 ? bn / 2.0 : 125.0;
-            // every additional slice adds the whole f32 output once more into L2 (measured: 13 us per slice on a
-            // 32000 x 768 output, i.e. about 1e-3 cycles per output element and slice)
-            double cost = (double)waves * (double)kb * (4.0 * mma + 60.0) + epi +
-                          (sp > 1 ? 300.0 * sp + (double)(sp - 1) * (double)m * (double)n * 1.0e-3 : 0.0);
-            if (bn == 256 && sp == 1 && m > 128) {
-                // unsplit 256-wide tiles may run with a split tail (see mcb_tc_gemm): same estimate as there
-                const long long workers = ctx->sm_count / 2, t256 = ((m + 255) / 256) * ((n + 255) / 256), rem = t256 % workers;
-                long long st = rem > 0 ? workers / rem : 1;
-                if (st > 8) st = 8;
-                if (st > kb_total / 4) st = kb_total / 4;
-                if (t256 > workers && st >= 2) {
-                    const double tail = (double)((t256 / workers) * kb_total + (kb_total + st - 1) / st) * (4.0 * 128.0 + 60.0) + 12.0 * 256 +
-                                        (atomic_out ? 1000.0 : kFixCycles);
-                    if (tail < 0.9 * cost) cost = tail;
-                }
-            }
-            if (cost < best - 1e-9) {
-                best = cost;
-                best_bn = bn;
-                best_split = sp;
-            }
-        }
-    }
-    *bn_out = best_bn;
-    *split_out = best_split;
 }
 
 extern "C" mcb_status mcb_gemm_bf16(mcb_ctx *ctx, const void *a, int32_t a_mn_major, const void *b, int32_t b_mn_major,
@@ -1300,7 +1316,7 @@ extern "C" mcb_status mcb_gemm_lowp(mcb_ctx *ctx, int32_t in_dt, const void *a, 
     p.split_k = split_k;
     if (split_k <= 0) { // let the library choose; splitting is only possible with the accumulating epilogue
         int bn = 0, sp = 1;
-        mcb_tc_plan(ctx, m, n, k, accumulate != 0, accumulate != 0, 1, &bn, &sp);
+        mcb_tc_plan(ctx, m, n, k, accumulate != 0, out_dt == MCB_F32, 1, &bn, &sp);
         p.bn = bn;
         p.split_k = sp;
     }

@@ -53,7 +53,7 @@ struct TcGemmParams {
 };
 mcb_status mcb_tc_gemm(mcb_ctx *ctx, const TcGemmParams &p);
 // tile width and reduction split for an [m, n] output reduced over k (see gemm_tc.cu)
-void mcb_tc_plan(mcb_ctx *ctx, int64_t m, int64_t n, int64_t k, bool allow_split, bool atomic_out, int fixed_split, int *bn_out,
+void mcb_tc_plan(mcb_ctx *ctx, int64_t m, int64_t n, int64_t k, bool allow_split, bool f32_out, int fixed_split, int *bn_out,
                  int *split_out);
 
 // flash_attn.cu: fused 16-bit attention, head dimensions that are multiples of 16 up to 128

@@ -359,6 +359,22 @@ def test_tc_gemm_split_tail(ops, oracle, m, n, k, a_mn, b_mn):
     close(outs["1"][0], outs["0"][0], 2e-6)  # same products, another grouping of the f32 sums
 
 
+# the form that the planner picks (tile width, one CTA or two, slices of the reduction) on both sides of its lines: one row block and
+# one row more, few and many k-blocks per worker, reductions that are cut into slices (split_k = 0: the library chooses)
+@pytest.mark.parametrize("m,n,k", [(128, 776, 3072), (129, 776, 1288), (300, 1032, 72), (2048, 264, 4096), (2056, 3080, 1352), (264, 520, 8192)])
+def test_tc_gemm_planned_form(ops, oracle, m, n, k):
+    for a_mn, b_mn in ((0, 0), (0, 1), (1, 1)):
+        if a_mn and m % 8:
+            continue
+        a = randn(k, m) if a_mn else randn(m, k)
+        b = randn(k, n) if b_mn else randn(n, k)
+        ref, init = gemm_ref(oracle, a, a_mn, b, b_mn), randn(m, n)
+        close(ops.gemm_bf16(a, a_mn, b, b_mn, m, n, k, out_dt=0), ref, 2e-5)
+        close(ops.gemm_bf16(a, a_mn, b, b_mn, m, n, k, out_dt=0, accumulate=True, split_k=0, init=init), ref + init, 2e-5)
+        out16 = ops.gemm_bf16(a, a_mn, b, b_mn, m, n, k, out_dt=5)
+        assert np.abs(out16 - ref).max() <= np.abs(ref).max() * 2.0 ** -8
+
+
 def test_tc_gemm_bias_accumulate_splitk(ops, oracle):
     m, n, k = 768, 768, 4096
     a, b, bias = randn(k, m), randn(k, n), randn(n)  # weight-gradient shape: both operands MN-major
