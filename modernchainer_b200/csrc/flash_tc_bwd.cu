@@ -1,4 +1,4 @@
-// Fused attention backward on the tcgen05 tensor cores (bf16 / f16, head_dim 64): two kernels from one template and a third:
+// Fused attention backward on the tcgen05 tensor cores (bf16 / f16): two kernels from one template and a third:
 //   MODE 0 (dK, dV): one CTA per 128-key tile; K_j, V_j stay in shared memory, the query tiles stream through.
 //   MODE 1 (dQ)    : one CTA per 128-query tile; Q_i, dO_i stay, the key tiles stream through (recomputes S, dP, dS).
 //   flash_tc_dq_kernel: dQ += dS K from the dS tiles that MODE 0 leaves in a scratch buffer as it goes (32 KB per pair,
